@@ -362,14 +362,17 @@ typedef struct claw2_batch_instance {
 /* Launch configurations of the batched kernel the autotuner chooses from:
  * threads per CTA x resident CTAs per SM x tile edge, and the grid's form
  * (variants 0-9: a persistent grid of SMs x resident CTAs, each CTA walking a
- * contiguous run of tiles; 10-13: one CTA per tile). */
+ * contiguous run of tiles; 10-13: one CTA per tile; 14-16: one CTA per tile
+ * marching over its rows, acoustics solvers only). */
 CLAW2_EXPORT int claw2_batch_num_variants(void);
 /* Threads per CTA and resident CTAs per SM of variant v (for reporting). */
 CLAW2_EXPORT int claw2_batch_variant_info(int v, int* threads, int* ctas_per_sm);
-/* Tile edge (cells) of variant v: 29, 21 or 13; -1 for an invalid v.  The
+/* Tile edge (cells) of variant v: 29, 21 or 13, or for variants 14-16 the rows
+ * (28, 14, 7) of a tile of 28 columns; -1 for an invalid v.  The
  * descriptors passed with variant v must number the tiles of that edge. */
 CLAW2_EXPORT int claw2_batch_variant_tile(int v);
-/* Tiles of an mx x my instance for a tile edge of 29, 21 or 13 cells. */
+/* Tiles of an mx x my instance for a tile edge of 29, 21 or 13 cells, or for
+ * tiles of 28 columns by 28, 14 or 7 rows. */
 CLAW2_EXPORT int claw2_batch_tiles_for(int tile, int mx, int my, int* nbx, int* nby);
 /* Tiles of an mx x my instance with 29x29 tiles (variants 0-5). */
 CLAW2_EXPORT int claw2_batch_tiles(int mx, int my, int* nbx, int* nby);

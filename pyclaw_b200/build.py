@@ -2,12 +2,13 @@
 
     python -m pyclaw_b200.build          # or pyclaw_b200.build.build()
 
-Compiles csrc/claw2_capi.cu (the plain and batched steps, which include the
-tile kernels and Riemann solvers) and csrc/claw2_adjoint.cu (multi-shot
-acoustics and its adjoint) with nvcc for sm_100a only, without FMA contraction
-so that the step keeps the reference's rounding, as two objects compiled in
-parallel under pyclaw_b200/_build/, and links them into pyclaw_b200/libclaw2.so
-(in-tree, so the library travels with the source tree).
+Compiles the sources under csrc/ (claw2_capi.cu: the plain step and the C ABI;
+claw2_acoustics.cu: the unsplit acoustics step; claw2_batch.cu: the batched
+form; claw2_adjoint.cu: multi-shot acoustics and its adjoint) with nvcc for
+sm_100a only, without FMA contraction so that the step keeps the reference's
+rounding, as objects compiled in parallel under pyclaw_b200/_build/, and links
+them into pyclaw_b200/libclaw2.so (in-tree, so the library travels with the
+source tree).
 """
 import os
 import shutil
@@ -18,12 +19,18 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(HERE)
 LIB = os.path.join(HERE, "libclaw2.so")
 SRCS = [os.path.join(HERE, "csrc", "claw2_capi.cu"),
+        os.path.join(HERE, "csrc", "claw2_batch.cu"),
+        os.path.join(HERE, "csrc", "claw2_acoustics.cu"),
         os.path.join(HERE, "csrc", "claw2_adjoint.cu")]
 OBJDIR = os.path.join(HERE, "_build")
 DEPS = SRCS + [os.path.join(HERE, "csrc", "claw2_kernels.cuh"),
                os.path.join(HERE, "csrc", "claw2_devattr.h"),
                os.path.join(HERE, "csrc", "claw2_riemann.cuh"),
                os.path.join(HERE, "csrc", "claw2_light.cuh"),
+               os.path.join(HERE, "csrc", "claw2_march.cuh"),
+               os.path.join(HERE, "csrc", "claw2_exact.cuh"),
+               os.path.join(HERE, "csrc", "claw2_launch.cuh"),
+               os.path.join(HERE, "csrc", "claw2_host.h"),
                os.path.join(HERE, "csrc", "claw2_lean.cuh"),
                os.path.join(HERE, "csrc", "claw2_tma.cuh"),
                os.path.join(ROOT, "include", "claw2.h"),

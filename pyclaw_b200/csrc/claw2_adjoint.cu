@@ -2,8 +2,8 @@
 // hand-written adjoint of its unsplit step (include/claw2_adjoint.h).
 //
 // Forward.  A shot is one wavefield; all shots share aux = (rho, c) and dt.
-// claw2_shots_step runs the fused tile step (the light body of
-// claw2_light.cuh) with the shot as the third grid dimension.
+// claw2_shots_step runs the plain step's tile (claw2_march.cuh) with the shot
+// as the third grid dimension.
 //
 // Adjoint.  One step of the reference's unsplit method (step2.f90:92-248,
 // flux2.f90:104-206, limiter.f90:34-58, philim.f90:18-55) with the vc-acoustics
@@ -36,7 +36,8 @@
 #include "../../include/claw2_adjoint.h"
 #include "claw2_devattr.h"
 #include "claw2_kernels.cuh"
-#include "claw2_light.cuh"
+#include "claw2_launch.cuh"
+#include "claw2_march.cuh"
 
 namespace claw2 {
 namespace adj {
@@ -44,7 +45,7 @@ namespace adj {
 constexpr int AT = 27;        // cells per tile side: 32 lanes = interfaces i0-2 .. i0+AT+2
 constexpr int ANT = 256;      // 8 warps
 constexpr int AR = AT + 4;    // shared accumulators: the tile plus a two-cell ghost ring
-constexpr int FT = 29;        // forward tile (the plain step's unsplit tile)
+constexpr int FT = 29;        // tile edge that the forward's scratch is counted in
 #ifndef CLAW2_ADJ_MINB
 #define CLAW2_ADJ_MINB 2      // resident CTAs per SM the register budget is sized for
 #endif
@@ -503,25 +504,20 @@ __global__ void __launch_bounds__(ANT, CLAW2_ADJ_MINB) adjoint_kernel(AdjArgs a)
 }
 
 // ---------------------------------------------------------------------------
-// forward: the plain tile step with the shot as third grid dimension
+// forward: the plain step's tile with the shot as third grid dimension
 // ---------------------------------------------------------------------------
-#ifndef CLAW2_LIGHT_MINB
-#define CLAW2_LIGHT_MINB 3
-#endif
-__global__ void __launch_bounds__(256, CLAW2_LIGHT_MINB) shots_step_kernel(StepArgs common, long long qstride)
+__global__ void __launch_bounds__(MARCH_NT, MarchVc::MINB) shots_step_kernel(StepArgs common, long long qstride, int rows)
 {
-    extern __shared__ double smem_dyn[];
-    DevCtx ctx{smem_dyn};
     const int shot = blockIdx.z;
     StepArgs a = common;
     a.qin += shot * qstride;
     a.qout += shot * qstride;
-    a.partials += (long long)shot * gridDim.x * gridDim.y;
+    a.partials += shot;                       // the shot's CFL cell
     a.ticket += shot;
     a.cfl_out += shot;
     const TileId t{(int)blockIdx.x, (int)blockIdx.y, (int)gridDim.x, (int)gridDim.y,
                    (int)(blockIdx.y * gridDim.x + blockIdx.x), (int)(gridDim.x * gridDim.y)};
-    light_tile_at<RpVcAcoustics, FT, FT, 256>(a, ctx, t);
+    march_tile<RpVcAcoustics, true>(a, t, rows);
 }
 
 struct ShotIO {
@@ -699,12 +695,10 @@ int claw2_shots_step(const claw2_problem* p, int nshots, long long shot_stride, 
     a.ticket = static_cast<unsigned int*>(scratch);
     a.partials = reinterpret_cast<double*>(static_cast<char*>(scratch) + tickets);
     a.cfl_out = cfl_dev;
-    using SM = LightSmem<FT, FT, 256>;
-    static std::atomic<uint64_t> optin{0};
-    if (smem_optin(optin, shots_step_kernel, SM::bytes) != cudaSuccess) return CLAW2_ERR_CUDA;
-    int nbx, nby;
-    ftiles(p, &nbx, &nby);
-    shots_step_kernel<<<dim3(nbx, nby, nshots), 256, SM::bytes, Sx(stream)>>>(a, shot_stride);
+    const int cols = (p->mx + MARCH_TX - 1) / MARCH_TX;
+    const int rows = march_rows_per_cta(p->rp, (long long)cols * nshots, p->my);
+    const dim3 grid(cols, (p->my + rows - 1) / rows, nshots);
+    shots_step_kernel<<<grid, MARCH_NT, 0, Sx(stream)>>>(a, shot_stride, rows);
     return cudaGetLastError() == cudaSuccess ? CLAW2_OK : CLAW2_ERR_CUDA;
 }
 

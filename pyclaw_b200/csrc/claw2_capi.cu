@@ -17,8 +17,9 @@
 #define CLAW2_EXPORT __attribute__((visibility("default")))
 #include "../../include/claw2.h"
 #include "claw2_devattr.h"
+#include "claw2_host.h"
 #include "claw2_kernels.cuh"
-#include "claw2_light.cuh"
+#include "claw2_launch.cuh"
 #include "claw2_lean.cuh"
 
 namespace claw2 {
@@ -27,41 +28,6 @@ namespace claw2 {
 #define CLAW2_MINB 2        // resident CTAs per SM the register budget is sized for
 #endif
 
-// Chained steps (launch_step with chained set): once every CTA of this step
-// has started, the next step's CTAs may start on the SMs this step frees;
-// each waits here until the step before it has completed and its writes are
-// visible.  In a kernel launched without the attribute both instructions
-// return at once.
-__device__ __forceinline__ void chain_wait()
-{
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-}
-
-// Launch kern, as a programmatic dependent of the previous kernel in the
-// stream when chained is set (the kernel calls chain_wait before it reads
-// anything).
-template <class... KArgs, class... Args>
-int launch_kernel(void (*kern)(KArgs...), dim3 grid, int threads, int smem, cudaStream_t st, bool chained,
-                  Args... args)
-{
-    if (!chained) {
-        kern<<<grid, threads, smem, st>>>(args...);
-        return cudaGetLastError() == cudaSuccess ? CLAW2_OK : CLAW2_ERR_CUDA;
-    }
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = dim3(threads);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kern, args...) == cudaSuccess ? CLAW2_OK : CLAW2_ERR_CUDA;
-}
-
 template <class RP, int TX, int TY, int NT, bool SPLIT>
 __global__ void __launch_bounds__(NT, CLAW2_MINB) step_kernel(StepArgs a)
 {
@@ -69,37 +35,6 @@ __global__ void __launch_bounds__(NT, CLAW2_MINB) step_kernel(StepArgs a)
     extern __shared__ double smem_dyn[];
     DevCtx ctx{smem_dyn};
     step_tile<RP, TX, TY, NT, SPLIT>(a, ctx);
-}
-
-// The two-wave acoustics solvers have a leaner unsplit body (claw2_light.cuh)
-// that needs fewer registers and less shared memory, so more CTAs fit per SM.
-template <class RP> struct HasLight { static constexpr bool value = false; };
-template <> struct HasLight<RpAcoustics> { static constexpr bool value = true; };
-template <> struct HasLight<RpVcAcoustics> { static constexpr bool value = true; };
-
-#ifndef CLAW2_LIGHT_MINB
-#define CLAW2_LIGHT_MINB 3
-#endif
-
-// Grids with fewer 29x29 tiles than a B200 has SMs leave most of the GPU idle
-// for the whole step; they run the light body on 13x13 tiles instead (4 to 5
-// times the CTAs; a line still has 32 lanes, of which 16 are used).
-constexpr int LIGHT_SMALL_TILE = 13, LIGHT_SMALL_GRID_TILES = 148;
-
-CLAW2_HD bool light_small_grid(int mx, int my)
-{
-    return (long long)((mx + 28) / 29) * (long long)((my + 28) / 29) < LIGHT_SMALL_GRID_TILES;
-}
-
-template <class RP, int T>
-__global__ void __launch_bounds__(256, CLAW2_LIGHT_MINB) light_step_kernel(StepArgs a)
-{
-    chain_wait();
-    extern __shared__ double smem_dyn[];
-    DevCtx ctx{smem_dyn};
-    const TileId t{(int)blockIdx.x, (int)blockIdx.y, (int)gridDim.x, (int)gridDim.y,
-                   (int)(blockIdx.y * gridDim.x + blockIdx.x), (int)(gridDim.x * gridDim.y)};
-    light_tile_at<RP, T, T, 256>(a, ctx, t);
 }
 
 // The dense-wave solvers without aux arrays (Euler, shallow water) have the
@@ -133,143 +68,6 @@ lean_step_kernel(StepArgs a, const __grid_constant__ CUtensorMap tm0, const __gr
     const TileId t{(int)blockIdx.x, (int)blockIdx.y, (int)gridDim.x, (int)gridDim.y,
                    (int)(blockIdx.y * gridDim.x + blockIdx.x), (int)(gridDim.x * gridDim.y)};
     lean_tile_at<RP, LTX, LTY, NT>(a, ctx, t, &tm0, &tm1, &halo_bar);
-}
-
-// Instance of tile t: the last one with tile_begin <= t (binary search).
-// With tb (the instances' tile_begin copied into shared memory by the
-// kernel) the search reads shared memory instead of walking the descriptors
-// in global memory, a chain of dependent L2 loads per tile.
-__device__ __forceinline__ int batch_instance_of(const claw2_batch_instance* __restrict__ inst, int ninst, int t,
-                                                 const int* tb = nullptr)
-{
-    int lo = 0, hi = ninst - 1;
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if ((tb ? tb[mid] : __ldg(&inst[mid].tile_begin)) <= t) lo = mid;
-        else hi = mid - 1;
-    }
-    return lo;
-}
-
-// batches of at most this many instances keep their tile_begin table in
-// shared memory (4 bytes each)
-constexpr int kBatchTableMax = 4096;
-
-// Instance of tile t + 1 given k, the instance of tile t: tile_begin is
-// non-decreasing, so it is the last instance at or after k whose tile_begin is
-// <= t + 1 (the same one or, crossing an instance's last tile, the next one
-// with tiles).
-__device__ __forceinline__ int batch_instance_after(const claw2_batch_instance* __restrict__ inst, int ninst, int k,
-                                                    int t, const int* tb)
-{
-    while (k + 1 < ninst && (tb ? tb[k + 1] : __ldg(&inst[k + 1].tile_begin)) <= t + 1) k++;
-    return k;
-}
-
-// Ask L2 for the input halo of tile t (instance k; rows j0-2..j0+TY+1 and
-// columns i0-2..i0+TX+1, clipped to the ghosted arrays, of the current state
-// and of aux) while the CTA works on the tile before it: an instance's data is
-// read once per step, from HBM, so the tile's first loads would otherwise wait
-// for DRAM.  One prefetch per 128-byte line, spread over the CTA's threads.
-// The addresses stay inside the instance's arrays; results do not depend on
-// it.
-template <int MEQN, int MAUX, int TX, int TY, int NT>
-__device__ __forceinline__ void batch_prefetch_tile(const claw2_batch_instance* __restrict__ inst, int k, int t)
-{
-    const claw2_batch_instance& I = inst[k];
-    const claw2_control* c = I.ctrl;
-    if (c->done) return;
-    const double* q = c->cur ? I.q1 : I.q0;
-    const int lt = t - I.tile_begin;
-    const int i0 = (lt % I.nbx) * TX, j0 = (lt / I.nbx) * TY;
-    const int rlo = j0 - 2, rhi = (j0 + TY + 1 < I.my + 1) ? j0 + TY + 1 : I.my + 1;
-    const int clo = i0 - 2, chi = (i0 + TX + 1 < I.mx + 1) ? i0 + TX + 1 : I.mx + 1;
-    // byte range of one row segment, in whole 128-byte lines
-    const long long b0 = (long long)(clo + CLAW2_NUM_GHOST) * 8, b1 = (long long)(chi + CLAW2_NUM_GHOST) * 8 + 8;
-    const int l0 = (int)(b0 >> 7), nl = (int)((b1 + 127) >> 7) - l0;
-    const int nrow = rhi - rlo + 1;
-    // one (field, row) per thread, its 128-byte lines in turn
-    for (int rf = threadIdx.x; rf < (MEQN + MAUX) * nrow; rf += NT) {
-        const int r = rf % nrow, f = rf / nrow;
-        const char* base = f < MEQN ? (const char*)(q + f * I.plane) : (const char*)(I.aux + (f - MEQN) * I.plane);
-        const char* row = base + (long long)(rlo + r + CLAW2_NUM_GHOST) * I.ld * 8 + ((long long)l0 << 7);
-        for (int line = 0; line < nl; line++) asm volatile("prefetch.global.L2 [%0];" ::"l"(row + (line << 7)));
-    }
-}
-
-// Batched step: a persistent grid walks the concatenated tile list of all
-// instances; each tile (T x T cells) is one tile-body call with that
-// instance's buffers, with an L2 prefetch of the CTA's next tile issued first.
-// body_doubles: the tile body's shared memory; with `table` set the
-// instances' tile_begin table follows it.
-template <class RP, int NT, int MINB, bool LIGHT, int T>
-__global__ void __launch_bounds__(NT, MINB)
-batch_kernel(const claw2_batch_instance* __restrict__ inst, int ninst, int ntiles, StepArgs common, int body_doubles,
-             int table)
-{
-    static_assert(LIGHT || T == 29, "the generic body runs 29x29 tiles in the batch");
-    extern __shared__ double smem_dyn[];
-    DevCtx ctx{smem_dyn};
-    int* tb = nullptr;
-    if (table) {
-        tb = reinterpret_cast<int*>(smem_dyn + body_doubles);
-        for (int i = threadIdx.x; i < ninst; i += NT) tb[i] = __ldg(&inst[i].tile_begin);
-        __syncthreads();
-    }
-    // each CTA takes a contiguous run of tiles: consecutive tiles mostly
-    // belong to the same instance (its descriptor and controller stay in L1)
-    // and share halo lines with the tile before them
-    const int tbeg = (int)((long long)ntiles * blockIdx.x / gridDim.x);
-    const int tend = (int)((long long)ntiles * (blockIdx.x + 1) / gridDim.x);
-    // the run's first instance by binary search, then one step at a time
-    int lo = tbeg < tend ? batch_instance_of(inst, ninst, tbeg, tb) : 0;
-    for (int t = tbeg; t < tend; t++) {
-        const int nxt = t + 1 < tend ? batch_instance_after(inst, ninst, lo, t, tb) : lo;
-        if (t + 1 < tend) batch_prefetch_tile<RP::MEQN, RP::MAUX, T, T, NT>(inst, nxt, t + 1);
-        const claw2_batch_instance& I = inst[lo];
-        StepArgs a = common;
-        a.q0 = I.q0; a.q1 = I.q1; a.aux = I.aux; a.ctrl = I.ctrl;
-        a.partials = I.partials; a.ticket = I.ticket;
-        a.ld = I.ld; a.plane = I.plane; a.mx = I.mx; a.my = I.my; a.dx = I.dx; a.dy = I.dy;
-        a.ghost_fused = (I.mx >= 4 && I.my >= 4) ? common.ghost_fused : 0;
-        const int lt = t - I.tile_begin;
-        const TileId tile{lt % I.nbx, lt / I.nbx, I.nbx, I.nby, lt, I.nbx * I.nby};
-        if constexpr (LIGHT) light_tile_at<RP, T, T, NT>(a, ctx, tile);
-        else step_tile_at<RP, 29, 29, NT, false>(a, ctx, tile);
-        __syncthreads();                            // shared memory is reused by the next tile
-        lo = nxt;
-    }
-}
-
-// Batched step with one CTA per tile (grid = all tiles of all instances):
-// the hardware hands tiles to SMs as slots free up, so uneven tiles balance
-// themselves, and no loop state stays live across the tile body.  The tile's
-// instance comes from the caller's tile -> instance map when there is one,
-// else from a binary search over the descriptors (a chain of dependent L2
-// loads at the CTA's start); there is no L2 prefetch of a next tile, the
-// other resident CTAs cover the first loads.
-template <class RP, int NT, int MINB, bool LIGHT, int T>
-__global__ void __launch_bounds__(NT, MINB)
-batch_tile_kernel(const claw2_batch_instance* __restrict__ inst, int ninst, StepArgs common,
-                  const int32_t* __restrict__ tile_inst)
-{
-    static_assert(LIGHT || T == 29, "the generic body runs 29x29 tiles in the batch");
-    extern __shared__ double smem_dyn[];
-    DevCtx ctx{smem_dyn};
-    const int t = (int)blockIdx.x;
-    int k = tile_inst ? __ldg(&tile_inst[t]) : -1;  // the caller's map: one load
-    if (k < 0 || k >= ninst || t < inst[k].tile_begin || t - inst[k].tile_begin >= inst[k].nbx * inst[k].nby)
-        k = batch_instance_of(inst, ninst, t);      // no map, or an entry that does not hold tile t
-    const claw2_batch_instance& I = inst[k];
-    StepArgs a = common;
-    a.q0 = I.q0; a.q1 = I.q1; a.aux = I.aux; a.ctrl = I.ctrl;
-    a.partials = I.partials; a.ticket = I.ticket;
-    a.ld = I.ld; a.plane = I.plane; a.mx = I.mx; a.my = I.my; a.dx = I.dx; a.dy = I.dy;
-    a.ghost_fused = (I.mx >= 4 && I.my >= 4) ? common.ghost_fused : 0;
-    const int lt = t - I.tile_begin;
-    const TileId tile{lt % I.nbx, lt / I.nbx, I.nbx, I.nby, lt, I.nbx * I.nby};
-    if constexpr (LIGHT) light_tile_at<RP, T, T, NT>(a, ctx, tile);
-    else step_tile_at<RP, 29, 29, NT, false>(a, ctx, tile);
 }
 
 // Tile shapes: a line of a chunk has 32 interface slots, so TX+3, TY+3 <= 32.
@@ -457,30 +255,12 @@ using namespace claw2;
 // ===========================================================================
 namespace {
 
-inline cudaStream_t S(void* s) { return reinterpret_cast<cudaStream_t>(s); }
-
-int solver_shape(int rp, int* meqn, int* mw, int* maux)
+// Problems stepped by the marching body (launch_step): the unsplit acoustics
+// solvers without capacity or f-waves.
+bool march_body(const claw2_problem* p)
 {
-    switch (rp) {
-    case CLAW2_RP_ACOUSTICS: *meqn = 3; *mw = 2; *maux = 0; return 0;
-    case CLAW2_RP_VC_ACOUSTICS: *meqn = 3; *mw = 2; *maux = 2; return 0;
-    case CLAW2_RP_EULER_4WAVE: *meqn = 4; *mw = 4; *maux = 0; return 0;
-    case CLAW2_RP_EULER_5WAVE: *meqn = 5; *mw = 5; *maux = 0; return 0;
-    case CLAW2_RP_SHALLOW_ROE: *meqn = 3; *mw = 3; *maux = 0; return 0;
-    case CLAW2_RP_PSYSTEM: *meqn = 3; *mw = 2; *maux = 4; return 0;
-    default: return -1;
-    }
-}
-
-bool periodic_ok(int bl, int bu) { return (bl == CLAW2_BC_PERIODIC) == (bu == CLAW2_BC_PERIODIC); }
-
-bool fused_ghosts(const claw2_problem* p)
-{
-    for (int d = 0; d < 2; d++) {
-        if (p->bc_lower[d] == CLAW2_BC_CUSTOM || p->bc_upper[d] == CLAW2_BC_CUSTOM) return false;
-        if (!periodic_ok(p->bc_lower[d], p->bc_upper[d])) return false;
-    }
-    return p->mx >= 4 && p->my >= 4;
+    return p->transverse >= 0 && p->index_capa < 0 && !p->use_fwave &&
+           (p->rp == CLAW2_RP_ACOUSTICS || p->rp == CLAW2_RP_VC_ACOUSTICS);
 }
 
 // Problems stepped by the lean body (launch_step_t): unsplit Euler and
@@ -491,14 +271,20 @@ bool lean_body(const claw2_problem* p)
            (p->rp == CLAW2_RP_EULER_4WAVE || p->rp == CLAW2_RP_EULER_5WAVE || p->rp == CLAW2_RP_SHALLOW_ROE);
 }
 
+// The tiles that claw2_scratch_bytes counts for it: 29x29 cells, 13x13 on
+// grids of fewer than 148 such tiles.
+constexpr int MARCH_SMALL_TILE = 13;
+bool march_small_grid(int mx, int my)
+{
+    return (long long)((mx + 28) / 29) * (long long)((my + 28) / 29) < 148;
+}
+
 void tiles(const claw2_problem* p, int* nbx, int* nby)
 {
     const bool split = p->transverse < 0;
     int tx = split ? STX : UTX, ty = split ? STY : UTY;
-    // the light body's choice for small grids (launch_light)
-    const bool light = !split && p->index_capa < 0 && !p->use_fwave &&
-                       (p->rp == CLAW2_RP_ACOUSTICS || p->rp == CLAW2_RP_VC_ACOUSTICS);
-    if (light && light_small_grid(p->mx, p->my)) tx = ty = LIGHT_SMALL_TILE;
+    // the marching body counts in tiles only for the scratch it is given
+    if (march_body(p) && march_small_grid(p->mx, p->my)) tx = ty = MARCH_SMALL_TILE;
     // the lean body's tiles (launch_step_t)
     if (lean_body(p)) { tx = LTX; ty = LTY; }
     *nbx = (p->mx + tx - 1) / tx;
@@ -519,44 +305,6 @@ void set_scratch(void* scratch, StepArgs& a)
 {
     a.ticket = static_cast<unsigned int*>(scratch);
     a.partials = reinterpret_cast<double*>(static_cast<char*>(scratch) + 64);
-}
-
-void fill_args(const claw2_problem* p, double* q, StepArgs& a)
-{
-    claw2_layout L;
-    claw2_get_layout(p, &L);
-    std::memset(&a, 0, sizeof a);
-    a.ld = L.ld; a.plane = L.plane;
-    a.mx = p->mx; a.my = p->my;
-    a.dx = p->dx; a.dy = p->dy;
-    a.order = p->order; a.trans = p->transverse; a.capa = p->index_capa; a.fwave = p->use_fwave;
-    a.limit_any = 0;
-    for (int w = 0; w < CLAW2_MAX_WAVES; w++) {
-        a.mthlim[w] = w < p->num_waves ? p->mthlim[w] : 0;
-        if (w < p->num_waves && p->mthlim[w] > 0) a.limit_any = 1;
-    }
-    for (int k = 0; k < CLAW2_MAX_PARAMS; k++) a.prm[k] = p->params[k];
-    a.ghost_fused = fused_ghosts(p) ? 1 : 0;
-    for (int d = 0; d < 2; d++) { a.bcl[d] = p->bc_lower[d]; a.bcu[d] = p->bc_upper[d]; }
-    (void)q;
-}
-
-template <class RP, int T>
-int launch_light_t(const StepArgs& a, int nbx, int nby, cudaStream_t st, bool chained)
-{
-    using SM = LightSmem<T, T, 256>;
-    auto kern = light_step_kernel<RP, T>;
-    static std::atomic<uint64_t> optin{0};
-    if (smem_optin(optin, kern, SM::bytes) != cudaSuccess) return CLAW2_ERR_CUDA;
-    return launch_kernel(kern, dim3(nbx, nby), 256, SM::bytes, st, chained, a);
-}
-
-// nbx x nby come from tiles(), which makes the same choice
-template <class RP>
-int launch_light(const StepArgs& a, int nbx, int nby, cudaStream_t st, bool chained)
-{
-    if (light_small_grid(a.mx, a.my)) return launch_light_t<RP, LIGHT_SMALL_TILE>(a, nbx, nby, st, chained);
-    return launch_light_t<RP, 29>(a, nbx, nby, st, chained);
 }
 
 // cuTensorMapEncodeTiled from the driver, found through the runtime (no link
@@ -626,8 +374,6 @@ int launch_lean(const StepArgs& a, int nbx, int nby, cudaStream_t st, bool chain
 template <class RP, bool SPLIT>
 int launch_step_t(const StepArgs& a, int nbx, int nby, cudaStream_t st, bool chained)
 {
-    if constexpr (!SPLIT && HasLight<RP>::value)
-        if (a.capa < 0 && !a.fwave) return launch_light<RP>(a, nbx, nby, st, chained);
     if constexpr (!SPLIT && HasLean<RP>::value)
         if (a.capa < 0 && !a.fwave) return launch_lean<RP>(a, nbx, nby, st, chained);
     constexpr int TX = SPLIT ? STX : UTX, TY = SPLIT ? STY : UTY, NT = SPLIT ? SNT : UNT;
@@ -642,6 +388,7 @@ int launch_step_t(const StepArgs& a, int nbx, int nby, cudaStream_t st, bool cha
 // device loop, so this step may overlap its end (launch_kernel).
 int launch_step(const claw2_problem* p, const StepArgs& a, cudaStream_t st, bool chained = false)
 {
+    if (march_body(p)) return launch_march(p->rp, a, st, chained);
     int nbx, nby;
     tiles(p, &nbx, &nby);
     const bool split = p->transverse < 0;
@@ -1012,217 +759,6 @@ int claw2_device_to_ref(const claw2_problem* p, int ncomp, const double* dev, do
 {
     if (!p || !ref || !dev || ncomp < 1) return CLAW2_ERR_INVALID;
     return conv(p, ncomp, dev, ref, false, true, S(stream));
-}
-
-// ---------------------------------------------------------------------------
-// batched form
-// ---------------------------------------------------------------------------
-}  // extern "C"
-
-namespace {
-// threads per CTA, resident CTAs per SM, tile edge (cells per CTA per work
-// item = tile^2).  Variants 4.. exist for the light acoustics body only
-// (claw2_batch_advance returns CLAW2_ERR_UNSUPPORTED for them with the other
-// solvers); a line of the light body has 32 lanes for tile + 3 interfaces, so
-// smaller tiles leave lanes idle but waste fewer cells at instance edges.
-// persistent: a grid of SMs x resident CTAs walking contiguous runs of tiles
-// (batch_kernel); otherwise one CTA per tile (batch_tile_kernel)
-struct BatchVariant { int threads, minb, tile, persistent; };
-constexpr BatchVariant kBatchVariants[] = {{256, 2, 29, 1}, {128, 4, 29, 1}, {128, 3, 29, 1}, {512, 1, 29, 1},
-                                           {256, 3, 29, 1}, {256, 4, 29, 1}, {256, 3, 21, 1}, {256, 4, 21, 1},
-                                           {256, 3, 13, 1}, {256, 4, 13, 1}, {256, 3, 29, 0}, {256, 4, 29, 0},
-                                           {128, 6, 29, 0}, {512, 2, 29, 0}};
-constexpr int kNumBatchVariants = sizeof(kBatchVariants) / sizeof(kBatchVariants[0]);
-
-bool batch_tile_ok(int tile) { return tile == 29 || tile == 21 || tile == 13; }
-
-template <class RP, int NT, int MINB, bool LIGHT, int T>
-int batch_launch_t(const StepArgs& common, const claw2_batch_instance* inst, int ninst, int ntiles, int nsteps,
-                   cudaStream_t st)
-{
-    constexpr int SMB = LIGHT ? LightSmem<T, T, NT>::bytes : TileSmem<RP, 29, 29, NT, false>::bytes;
-    constexpr int kSmemLimit = 227 * 1024;        // dynamic shared memory a CTA can opt in to
-    constexpr int SMMAX = SMB + 4 * kBatchTableMax < kSmemLimit ? SMB + 4 * kBatchTableMax : SMB;
-    auto kern = batch_kernel<RP, NT, MINB, LIGHT, T>;
-    static std::atomic<uint64_t> optin{0};
-    if (smem_optin(optin, kern, SMMAX) != cudaSuccess) return CLAW2_ERR_CUDA;
-    // the persistent grid: SMs x the CTAs that fit with this launch's table
-    const int tbytes = (4 * ninst + 15) / 16 * 16;
-    const int table = ninst <= kBatchTableMax && SMB + tbytes <= SMMAX;
-    const int smem = SMB + (table ? tbytes : 0);
-    int dev = 0, nsm = 0, occ = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, NT, smem) != cudaSuccess || occ < 1)
-        return CLAW2_ERR_CUDA;
-    const int grid = nsm * occ;
-    const int g = ntiles < grid ? ntiles : grid;
-    for (int n = 0; n < nsteps; n++) {
-        kern<<<g, NT, smem, st>>>(inst, ninst, ntiles, common, SMB / 8, table);
-        if (cudaGetLastError() != cudaSuccess) return CLAW2_ERR_CUDA;
-    }
-    return CLAW2_OK;
-}
-
-template <class RP, int NT, int MINB, bool LIGHT, int T>
-int batch_launch_tiles(const StepArgs& common, const claw2_batch_instance* inst, int ninst, int ntiles, int nsteps,
-                       const int32_t* tile_inst, cudaStream_t st)
-{
-    constexpr int SMB = LIGHT ? LightSmem<T, T, NT>::bytes : TileSmem<RP, 29, 29, NT, false>::bytes;
-    auto kern = batch_tile_kernel<RP, NT, MINB, LIGHT, T>;
-    static std::atomic<uint64_t> optin{0};
-    if (smem_optin(optin, kern, SMB) != cudaSuccess) return CLAW2_ERR_CUDA;
-    for (int n = 0; n < nsteps; n++) {
-        kern<<<ntiles, NT, SMB, st>>>(inst, ninst, common, tile_inst);
-        if (cudaGetLastError() != cudaSuccess) return CLAW2_ERR_CUDA;
-    }
-    return CLAW2_OK;
-}
-
-template <class RP>
-int batch_launch_rp(int variant, const StepArgs& c, const claw2_batch_instance* inst, int ninst, int ntiles,
-                    int nsteps, const int32_t* tile_inst, cudaStream_t st)
-{
-    if constexpr (HasLight<RP>::value) {
-        if (c.capa < 0 && !c.fwave) {
-            switch (variant) {
-            case 0: return batch_launch_t<RP, 256, 2, true, 29>(c, inst, ninst, ntiles, nsteps, st);
-            case 1: return batch_launch_t<RP, 128, 4, true, 29>(c, inst, ninst, ntiles, nsteps, st);
-            case 2: return batch_launch_t<RP, 128, 3, true, 29>(c, inst, ninst, ntiles, nsteps, st);
-            case 3: return batch_launch_t<RP, 512, 1, true, 29>(c, inst, ninst, ntiles, nsteps, st);
-            case 4: return batch_launch_t<RP, 256, 3, true, 29>(c, inst, ninst, ntiles, nsteps, st);
-            case 5: return batch_launch_t<RP, 256, 4, true, 29>(c, inst, ninst, ntiles, nsteps, st);
-            case 6: return batch_launch_t<RP, 256, 3, true, 21>(c, inst, ninst, ntiles, nsteps, st);
-            case 7: return batch_launch_t<RP, 256, 4, true, 21>(c, inst, ninst, ntiles, nsteps, st);
-            case 8: return batch_launch_t<RP, 256, 3, true, 13>(c, inst, ninst, ntiles, nsteps, st);
-            case 9: return batch_launch_t<RP, 256, 4, true, 13>(c, inst, ninst, ntiles, nsteps, st);
-            case 10: return batch_launch_tiles<RP, 256, 3, true, 29>(c, inst, ninst, ntiles, nsteps, tile_inst, st);
-            case 11: return batch_launch_tiles<RP, 256, 4, true, 29>(c, inst, ninst, ntiles, nsteps, tile_inst, st);
-            case 12: return batch_launch_tiles<RP, 128, 6, true, 29>(c, inst, ninst, ntiles, nsteps, tile_inst, st);
-            case 13: return batch_launch_tiles<RP, 512, 2, true, 29>(c, inst, ninst, ntiles, nsteps, tile_inst, st);
-            default: return CLAW2_ERR_INVALID;
-            }
-        }
-    }
-    switch (variant) {
-    case 0: return batch_launch_t<RP, 256, 2, false, 29>(c, inst, ninst, ntiles, nsteps, st);
-    case 1: return batch_launch_t<RP, 128, 4, false, 29>(c, inst, ninst, ntiles, nsteps, st);
-    case 2: return batch_launch_t<RP, 128, 3, false, 29>(c, inst, ninst, ntiles, nsteps, st);
-    case 3: return batch_launch_t<RP, 512, 1, false, 29>(c, inst, ninst, ntiles, nsteps, st);
-    default: return variant < kNumBatchVariants ? CLAW2_ERR_UNSUPPORTED : CLAW2_ERR_INVALID;
-    }
-}
-
-int batch_launch(const claw2_problem* p, const claw2_batch_instance* inst, int ninst, int ntiles, int nsteps,
-                 int variant, const int32_t* tile_inst, cudaStream_t st)
-{
-    StepArgs c;
-    fill_args(p, nullptr, c);
-    c.ghost_fused = 1;
-    for (int d = 0; d < 2; d++)
-        if (p->bc_lower[d] == CLAW2_BC_CUSTOM || p->bc_upper[d] == CLAW2_BC_CUSTOM) return CLAW2_ERR_UNSUPPORTED;
-    switch (p->rp) {
-    case CLAW2_RP_ACOUSTICS: return batch_launch_rp<RpAcoustics>(variant, c, inst, ninst, ntiles, nsteps, tile_inst, st);
-    case CLAW2_RP_VC_ACOUSTICS: return batch_launch_rp<RpVcAcoustics>(variant, c, inst, ninst, ntiles, nsteps, tile_inst, st);
-    case CLAW2_RP_EULER_4WAVE: return batch_launch_rp<RpEuler<false>>(variant, c, inst, ninst, ntiles, nsteps, tile_inst, st);
-    case CLAW2_RP_EULER_5WAVE: return batch_launch_rp<RpEuler<true>>(variant, c, inst, ninst, ntiles, nsteps, tile_inst, st);
-    case CLAW2_RP_SHALLOW_ROE: return batch_launch_rp<RpShallow>(variant, c, inst, ninst, ntiles, nsteps, tile_inst, st);
-    case CLAW2_RP_PSYSTEM: return batch_launch_rp<RpPsystem>(variant, c, inst, ninst, ntiles, nsteps, tile_inst, st);
-    default: return CLAW2_ERR_INVALID;
-    }
-}
-
-int batch_check(const claw2_problem* p, const claw2_batch_instance* inst, int ninst, int ntiles, int nsteps,
-                int variant)
-{
-    if (!p || !inst || ninst < 1 || ntiles < 1 || nsteps < 0) return CLAW2_ERR_INVALID;
-    if (variant < 0 || variant >= kNumBatchVariants) return CLAW2_ERR_INVALID;
-    if (p->transverse < 0) return CLAW2_ERR_UNSUPPORTED;
-    int meqn, mw, maux;
-    if (solver_shape(p->rp, &meqn, &mw, &maux) || p->num_eqn != meqn || p->num_waves != mw || p->num_aux < maux)
-        return CLAW2_ERR_INVALID;
-    if (p->num_ghost != CLAW2_NUM_GHOST || p->index_capa >= p->num_aux) return CLAW2_ERR_INVALID;
-    for (int d = 0; d < 2; d++)
-        if (!periodic_ok(p->bc_lower[d], p->bc_upper[d])) return CLAW2_ERR_UNSUPPORTED;
-    return CLAW2_OK;
-}
-}  // namespace
-
-extern "C" {
-
-int claw2_batch_num_variants(void) { return kNumBatchVariants; }
-
-int claw2_batch_variant_info(int v, int* threads, int* ctas_per_sm)
-{
-    if (v < 0 || v >= kNumBatchVariants || !threads || !ctas_per_sm) return CLAW2_ERR_INVALID;
-    *threads = kBatchVariants[v].threads;
-    *ctas_per_sm = kBatchVariants[v].minb;
-    return CLAW2_OK;
-}
-
-int claw2_batch_tiles(int mx, int my, int* nbx, int* nby)
-{
-    return claw2_batch_tiles_for(UTX, mx, my, nbx, nby);
-}
-
-int claw2_batch_variant_tile(int v)
-{
-    if (v < 0 || v >= kNumBatchVariants) return -1;
-    return kBatchVariants[v].tile;
-}
-
-int claw2_batch_tiles_for(int tile, int mx, int my, int* nbx, int* nby)
-{
-    if (!batch_tile_ok(tile) || mx < 4 || my < 4 || !nbx || !nby) return CLAW2_ERR_INVALID;
-    *nbx = (mx + tile - 1) / tile;
-    *nby = (my + tile - 1) / tile;
-    return CLAW2_OK;
-}
-
-int claw2_batch_advance(const claw2_problem* p, const claw2_batch_instance* inst, int ninst, int ntiles, int nsteps,
-                        int variant, void* stream)
-{
-    return claw2_batch_advance_map(p, inst, ninst, ntiles, nullptr, nsteps, variant, stream);
-}
-
-int claw2_batch_advance_map(const claw2_problem* p, const claw2_batch_instance* inst, int ninst, int ntiles,
-                            const int32_t* tile_inst, int nsteps, int variant, void* stream)
-{
-    int rc = batch_check(p, inst, ninst, ntiles, nsteps, variant);
-    if (rc) return rc;
-    return batch_launch(p, inst, ninst, ntiles, nsteps, variant, tile_inst, S(stream));
-}
-
-int claw2_batch_graph_create(const claw2_problem* p, const claw2_batch_instance* inst, int ninst, int ntiles,
-                             int nsteps, int variant, void** graph_exec)
-{
-    return claw2_batch_graph_create_map(p, inst, ninst, ntiles, nullptr, nsteps, variant, graph_exec);
-}
-
-int claw2_batch_graph_create_map(const claw2_problem* p, const claw2_batch_instance* inst, int ninst, int ntiles,
-                                 const int32_t* tile_inst, int nsteps, int variant, void** graph_exec)
-{
-    int rc = batch_check(p, inst, ninst, ntiles, nsteps, variant);
-    if (rc) return rc;
-    if (!graph_exec) return CLAW2_ERR_INVALID;
-    // one launch outside the capture configures the kernel (shared-memory
-    // attribute, occupancy) so that the capture itself only records launches
-    cudaStream_t st;
-    if (cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking) != cudaSuccess) return CLAW2_ERR_CUDA;
-    rc = batch_launch(p, inst, ninst, ntiles, 0, variant, tile_inst, st);
-    cudaGraph_t graph = nullptr;
-    cudaGraphExec_t exec = nullptr;
-    if (!rc && cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal) != cudaSuccess) rc = CLAW2_ERR_CUDA;
-    if (!rc) {
-        const int r2 = batch_launch(p, inst, ninst, ntiles, nsteps, variant, tile_inst, st);
-        if (cudaStreamEndCapture(st, &graph) != cudaSuccess || r2) rc = r2 ? r2 : CLAW2_ERR_CUDA;
-    }
-    if (!rc && cudaGraphInstantiate(&exec, graph, 0) != cudaSuccess) rc = CLAW2_ERR_CUDA;
-    if (graph) cudaGraphDestroy(graph);
-    cudaStreamDestroy(st);
-    if (rc) return rc;
-    *graph_exec = exec;
-    return CLAW2_OK;
 }
 
 int claw2_graph_launch(void* graph_exec, void* stream)

@@ -575,6 +575,75 @@ struct TileId {
     int bx, by, nbx, nby, part, ntiles;
 };
 
+// The step's CFL number (nf: 1 a non-finite state, 2 a tile's input never
+// arrived) goes to the controller or to cfl_out.
+template <class Ctx>
+CLAW2_HD void finish_step(const StepArgs& a, Ctx& ctx, double cfl, int nf)
+{
+    if (a.ctrl && !a.ctrl_readonly) control_update(a.ctrl, cfl, nf);
+    else if (a.ctrl_readonly) *a.cfl_out = nf ? 1.0 / 0.0 : cfl;
+    else *a.cfl_out = nf ? ctx.nan() : cfl;
+}
+
+// Block CFL max (deterministic: max is exact) and last-block epilogue: warp max
+// by shuffles, then one value per warp.  CFL numbers are >= 0; a NaN one
+// counts as a non-finite state, and -1 flags a warp that saw one; a tile that
+// could not be computed reports -2.  red: NT/32 + 1 doubles of shared memory.
+template <int NT, class Ctx>
+CLAW2_HD void report_cfl(const StepArgs& a, Ctx& ctx, const TileId& tile, double* red, double cflm, bool bad, bool fault)
+{
+    const int tid = ctx.tid();
+    {
+        const bool nfw = ctx.warp_any(bad || cflm != cflm);
+        const double mw = ctx.warp_max(cflm);
+        if ((tid & 31) == 0) red[tid >> 5] = nfw ? -1.0 : mw;
+    }
+    ctx.sync();
+    constexpr int NW = NT / 32;
+    if (tid == 0) {
+        double mxv = 0.0;
+        int nf = 0;
+        for (int t = 0; t < NW; t++) {
+            if (red[t] < 0.0) nf = 1;
+            else mxv = mxv > red[t] ? mxv : red[t];
+        }
+        a.partials[tile.part] = fault ? -2.0 : (nf ? -1.0 : mxv);
+        ctx.fence();
+        const unsigned int prev = ctx.atomic_inc(a.ticket);
+        red[NW] = prev == (unsigned int)(tile.ntiles - 1) ? 1.0 : 0.0;     // this CTA arrived last
+    }
+    ctx.sync();
+    if (red[NW] != 0.0) {
+        // the last CTA reduces every CTA's partial with all its threads
+        ctx.fence();
+        double cfl = 0.0;
+        bool nonfinite = false, lost = false;
+        for (int b = tid; b < tile.ntiles; b += NT) {
+            const double v = ctx.load_volatile(&a.partials[b]);
+            if (v < 0.0) nonfinite = true;
+            else cfl = cfl > v ? cfl : v;
+            if (v == -2.0) lost = true;
+        }
+        const bool nfw = ctx.warp_any(nonfinite);
+        const bool lw = ctx.warp_any(lost);
+        const double mw = ctx.warp_max(cfl);
+        if ((tid & 31) == 0) red[tid >> 5] = lw ? -2.0 : (nfw ? -1.0 : mw);
+        ctx.sync();
+        if (tid == 0) {
+            cfl = 0.0;
+            int nf = 0;
+            for (int t = 0; t < NW; t++) {
+                if (red[t] == -2.0) nf = 2;
+                else if (red[t] < 0.0 && nf == 0) nf = 1;
+                else if (red[t] >= 0.0) cfl = cfl > red[t] ? cfl : red[t];
+            }
+            finish_step(a, ctx, cfl, nf);
+            *a.ticket = 0u;
+            ctx.fence();
+        }
+    }
+}
+
 // Final values of the tile's cells (Qx: row stride TX, component stride QSTR,
 // row 0 = tile row j0) and their ghost images, then the block CFL max and the
 // last-arriving CTA's reduction over all CTAs (and, in controlled mode, the
@@ -659,61 +728,7 @@ CLAW2_HD void finish_tile(const StepArgs& a, Ctx& ctx, const TileId& tile, const
         }
     }
 
-    // ---- block CFL max (deterministic: max is exact) and last-block epilogue:
-    // warp max by shuffles, then one value per warp.  CFL numbers are >= 0; a
-    // NaN one counts as a non-finite state, and -1 flags a warp that saw one;
-    // a tile that could not be computed reports -2.
-    {
-        const bool nfw = ctx.warp_any(bad != 0 || cflm != cflm);
-        const double mw = ctx.warp_max(cflm);
-        if ((tid & 31) == 0) red[tid >> 5] = nfw ? -1.0 : mw;
-    }
-    ctx.sync();
-    constexpr int NW = NT / 32;
-    if (tid == 0) {
-        double mxv = 0.0;
-        int nf = 0;
-        for (int t = 0; t < NW; t++) {
-            if (red[t] < 0.0) nf = 1;
-            else mxv = mxv > red[t] ? mxv : red[t];
-        }
-        a.partials[tile.part] = fault ? -2.0 : (nf ? -1.0 : mxv);
-        ctx.fence();
-        const unsigned int prev = ctx.atomic_inc(a.ticket);
-        red[NW] = prev == (unsigned int)(tile.ntiles - 1) ? 1.0 : 0.0;     // this CTA arrived last
-    }
-    ctx.sync();
-    if (red[NW] != 0.0) {
-        // the last CTA reduces every CTA's partial with all its threads
-        ctx.fence();
-        double cfl = 0.0;
-        bool nonfinite = false, lost = false;
-        for (int b = tid; b < tile.ntiles; b += NT) {
-            const double v = ctx.load_volatile(&a.partials[b]);
-            if (v < 0.0) nonfinite = true;
-            else cfl = cfl > v ? cfl : v;
-            if (v == -2.0) lost = true;
-        }
-        const bool nfw = ctx.warp_any(nonfinite);
-        const bool lw = ctx.warp_any(lost);
-        const double mw = ctx.warp_max(cfl);
-        if ((tid & 31) == 0) red[tid >> 5] = lw ? -2.0 : (nfw ? -1.0 : mw);
-        ctx.sync();
-        if (tid == 0) {
-            cfl = 0.0;
-            int nf = 0;
-            for (int t = 0; t < NW; t++) {
-                if (red[t] == -2.0) nf = 2;
-                else if (red[t] < 0.0 && nf == 0) nf = 1;
-                else if (red[t] >= 0.0) cfl = cfl > red[t] ? cfl : red[t];
-            }
-            if (a.ctrl && !a.ctrl_readonly) control_update(a.ctrl, cfl, nf);
-            else if (a.ctrl_readonly) *a.cfl_out = nf ? 1.0 / 0.0 : cfl;
-            else *a.cfl_out = nf ? ctx.nan() : cfl;
-            *a.ticket = 0u;
-            ctx.fence();
-        }
-    }
+    report_cfl<NT>(a, ctx, tile, red, cflm, bad != 0, fault);
 }
 
 // f(IntC<0>{}), ..., f(IntC<N-1>{}): a loop whose index is a compile-time constant
