@@ -28,7 +28,9 @@ DEPS = SRCS + [os.path.join(HERE, "csrc", "claw2_kernels.cuh"),
                os.path.join(HERE, "csrc", "claw2_riemann.cuh"),
                os.path.join(HERE, "csrc", "claw2_light.cuh"),
                os.path.join(HERE, "csrc", "claw2_march.cuh"),
+               os.path.join(HERE, "csrc", "claw2_dense.cuh"),
                os.path.join(HERE, "csrc", "claw2_exact.cuh"),
+               os.path.join(HERE, "csrc", "claw2_limit.cuh"),
                os.path.join(HERE, "csrc", "claw2_launch.cuh"),
                os.path.join(HERE, "csrc", "claw2_host.h"),
                os.path.join(HERE, "csrc", "claw2_lean.cuh"),

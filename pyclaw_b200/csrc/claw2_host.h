@@ -50,6 +50,9 @@ inline void fill_args(const claw2_problem* p, double* q, StepArgs& a)
         a.mthlim[w] = w < p->num_waves ? p->mthlim[w] : 0;
         if (w < p->num_waves && p->mthlim[w] > 0) a.limit_any = 1;
     }
+    a.limit_first = a.mthlim[0];
+    for (int w = 1; w < 4 && w < p->num_waves; w++)
+        if (a.mthlim[w] != a.limit_first) a.limit_first = -1;
     for (int k = 0; k < CLAW2_MAX_PARAMS; k++) a.prm[k] = p->params[k];
     a.ghost_fused = fused_ghosts(p) ? 1 : 0;
     for (int d = 0; d < 2; d++) { a.bcl[d] = p->bc_lower[d]; a.bcu[d] = p->bc_upper[d]; }

@@ -51,6 +51,7 @@ struct StepArgs {
     double dx, dy, dt;
     int order, trans, capa, fwave, limit_any;
     int mthlim[CLAW2_MAX_WAVES];
+    int limit_first;       // limiter of the first min(waves, 4) waves if they share it, else -1
     double prm[CLAW2_MAX_PARAMS];
     int ghost_fused;
     int bcl[2], bcu[2];

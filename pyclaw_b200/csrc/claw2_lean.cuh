@@ -5,15 +5,20 @@
 // same operations in the same order, so the results are the same values; only
 // the data movement differs, as in the acoustics body of claw2_light.cuh:
 //  - each lane computes the quantities of one cell that the normal solve
-//    needs (RP::Cell: square roots, pressures, Roe-average numerators) and
+//    needs (dense_cell: square roots, pressures, Roe-average numerators) and
 //    takes those of the cell right of its interface from the next lane, so
 //    each cell's are computed once per line instead of once per interface;
 //    with TX = 28 the 32 lanes hold the 32 cells i0-2 .. i0+29 of the line's
 //    31 interfaces;
+//  - the solves are those of claw2_dense.cuh: the same bits from fewer
+//    instructions and no divergent divisions;
 //  - the normal solve stays in registers; for the limiter each lane takes its
-//    right neighbour's wave by warp shuffle and forms dotr = wave(k).wave(k+1);
-//    dotl of lane k is dotr of lane k-1 (one more shuffle), the same products
-//    summed in the same component order (a*b == b*a exactly);
+//    right neighbour's wave strengths and Roe averages by warp shuffle and forms
+//    dotr = wave(k).wave(k+1); dotl of lane k is dotr of lane k-1 (one more
+//    shuffle), the same products summed in the same component order (a*b ==
+//    b*a exactly);
+//  - a line whose cells hold one state carries no waves: its corrections and
+//    splits are passed over;
 //  - what the cell left of an interface needs from it (dtdx*amdq, fadd and
 //    the two transverse splits) moves one lane by shuffle;
 //  - a cell's own-line contributions stay in registers; only the two
@@ -27,8 +32,16 @@
 //  - a tile whose staged halo holds one state skips both sweeps: every
 //    interface would join two equal states, so its cells keep their values
 //    and its CFL number comes from one Riemann solve (uniform_cfl).
+//
+// Bound by the latency of the FP64 chains and by issue: 128 registers a thread
+// leave 4 warps per SM quarter, which issue 44% of the cycles (FP64 pipe 36%
+// busy; stalled on dependences 2.1 and barriers 1.4 of the 8 warp-cycles per
+// instruction).  Euler 4-wave, us a step on a B200: 1280 x 320 66.8 (75.4 with
+// the solves of claw2_riemann.cuh), 1500^2 283 (331), 256^2 29.9 (36.7); 5-wave
+// 1500^2 453 (532); shallow water 1500^2 292 (367), 256^2 22.5 (26.4).
 #pragma once
 
+#include "claw2_dense.cuh"
 #include "claw2_kernels.cuh"
 #include "claw2_tma.cuh"
 
@@ -64,10 +77,10 @@ __device__ __forceinline__ int lean_hidx(int m, int r, int c)
 // One chunk of one sweep direction (arguments as in sweep_chunk); CXb is the
 // half of the exchange array this chunk uses.
 template <class RP, int IXY, int TX, int TY, int NT, class Ctx>
-CLAW2_HD void lean_chunk(const StepArgs& a, Ctx& ctx, const double* H, double* Qx, double* CXb, int i0, int j0,
+__device__ __forceinline__ void lean_chunk(const StepArgs& a, Ctx& ctx, const double* H, double* Qx, double* CXb, int i0, int j0,
                          int line, int cfirst, int clast, bool lineok, double dtn, double dtt, double& cflm)
 {
-    constexpr int MEQN = RP::MEQN, MW = RP::MW, NROE = RP::NROE;
+    constexpr int MEQN = RP::MEQN, MW = RP::MW;
     using SM = LeanSmem<RP, TX, TY, NT>;
     constexpr int TR = SM::TR;
     // the staged input of cell (kk along the slice, ll across it)
@@ -84,108 +97,67 @@ CLAW2_HD void lean_chunk(const StepArgs& a, Ctx& ctx, const double* H, double* Q
     const bool ifok = lineok && slot < NSLOT && k <= len + 1;
     const bool lim = ifok && slot >= 1 && slot <= NSLOT - 2 && k >= 0 && k <= len;
 
-    // ---------------- normal solve ----------------
-    // the waves are kept as their strengths: wave p is alpha[p] times rpn2c's
-    // eigenvector of the Roe averages, rebuilt with the same operations where
-    // it is needed (RP::wave_of), and s[p] is RP::speed<p>(roe)
-    double alpha[MW], amdq[MEQN], apdq[MEQN], roe[NROE];
-#pragma unroll
-    for (int p = 0; p < MW; p++) alpha[p] = 0.0;
-#pragma unroll
-    for (int m = 0; m < MEQN; m++) { amdq[m] = 0.0; apdq[m] = 0.0; }
-#pragma unroll
-    for (int r = 0; r < NROE; r++) roe[r] = 0.0;
+    using D = typename DenseOf<RP>::type;
+    constexpr int NR = D::NR, NCD = D::NCD;
+    // interfaces whose fluxes and waves count, and whether this lane's is one
+    // (lim) or a limiter neighbour (ifok)
+    double al[MW], amdq[MEQN], apdq[MEQN], roe[NR], cqxx[MEQN], fadd[MEQN];
+    bool flat;
     {
         // this lane's cell k-1, and cell k from the next lane
-        typename RP::Cell L{};
-        double qL[MEQN];
+        double qL[MEQN], qR[MEQN], L[NCD], R[NCD];
         const bool cellok = lineok && k - 1 <= len + 1;
 #pragma unroll
-        for (int m = 0; m < MEQN; m++) qL[m] = cellok ? hq(m, k - 1, line) : 0.0;
-        if (cellok) L = RP::template cell<IXY>(qL, a.prm);
-        const typename RP::Cell R = L.map([&](double v) { return ctx.shfl_down(v); });
-        if (ifok) {
-            double qR[MEQN];
+        for (int m = 0; m < MEQN; m++) { qL[m] = hq(m, k - 1, line); qR[m] = hq(m, slot < 31 ? k : k - 1, line); }
+        dense_cell<D, IXY>(a, qL, cellok, L);
 #pragma unroll
-            for (int m = 0; m < MEQN; m++) qR[m] = hq(m, k, line);
-            RP::template rpn2a<IXY>(qL, qR, L, R, a.prm, alpha, amdq, apdq, roe);
-        }
+        for (int f = 0; f < NCD; f++) R[f] = f != D::S0 ? ctx.shfl_down(L[f]) : 0.0;
+        bool eq = true;
+#pragma unroll
+        for (int m = 0; m < MEQN; m++) eq = eq && qL[m] == qR[m];
+        flat = __all_sync(0xffffffffu, eq || !ifok);
+        dense_normal<D, IXY>(a, qL, qR, L, R, ifok, al, amdq, apdq, roe);
     }
 
     // ---------------- CFL, limiter, second-order corrections ----------------
     if (lim) {
-        static_for<MW>([&](auto P) {
-            const double sp = RP::template speed<decltype(P)::value>(roe);
-            const double c1 = dtn * sp, c2 = -dtn * sp;
-            cflm = cflm > c1 ? cflm : c1;
-            cflm = cflm > c2 ? cflm : c2;
-        });
+        const double c = fabs(dtn) * D::top_speed(roe);     // the largest of dtn s and -dtn s over the waves
+        cflm = cflm > c ? cflm : c;
     }
-    double cqxx[MEQN], fadd[MEQN];
-#pragma unroll
-    for (int m = 0; m < MEQN; m++) { cqxx[m] = 0.0; fadd[m] = 0.0; }
-    if (a.order == 2) {                       // uniform: every lane takes part in the shuffles
-        const double dtdxave = 0.5 * (dtn + dtn);
-        // the right neighbour's strengths and the Roe averages its waves use
-        double alr[MW], roer[NROE];
-#pragma unroll
-        for (int p = 0; p < MW; p++) alr[p] = ctx.shfl_down(alpha[p]);
-#pragma unroll
-        for (int r = 0; r < NROE; r++) roer[r] = r < RP::NROE_WAVE ? ctx.shfl_down(roe[r]) : 0.0;
-        static_for<MW>([&](auto P) {
-            constexpr int p = decltype(P)::value;
-            double wv[MEQN], wn[MEQN];
-            RP::template wave_of<IXY, p>(alpha[p], roe, wv);
-            RP::template wave_of<IXY, p>(alr[p], roer, wn);
-            // dotr = wave(k).wave(k+1); dotl of lane k is dotr of lane k-1
-            double dotr = 0.0;
-#pragma unroll
-            for (int m = 0; m < MEQN; m++) dotr = dotr + wv[m] * wn[m];
-            const double dotl = ctx.shfl_up(dotr);
-            const double sp = RP::template speed<p>(roe);
-            if (lim) {
-                const int meth = a.mthlim[p];
-                if (a.limit_any && meth != 0) {
-                    double wnorm2 = 0.0;
-#pragma unroll
-                    for (int m = 0; m < MEQN; m++) wnorm2 = wnorm2 + wv[m] * wv[m];
-                    if (wnorm2 != 0.0) {
-                        const double phi = philim(wnorm2, sp > 0.0 ? dotl : dotr, meth);
-#pragma unroll
-                        for (int m = 0; m < MEQN; m++) wv[m] = phi * wv[m];
-                    }
-                }
-                const double as = fabs(sp);
-                const double f = as * (1.0 - as * dtdxave);
-#pragma unroll
-                for (int m = 0; m < MEQN; m++) cqxx[m] = (p == 0) ? f * wv[m] : cqxx[m] + f * wv[m];
-            }
-        });
-#pragma unroll
-        for (int m = 0; m < MEQN; m++) fadd[m] = 0.5 * cqxx[m];
-    }
-
-    // ---------------- transverse splits ----------------
     double bmL[MEQN], bpL[MEQN], bmR[MEQN], bpR[MEQN];
 #pragma unroll
-    for (int m = 0; m < MEQN; m++) { bmL[m] = 0.0; bpL[m] = 0.0; bmR[m] = 0.0; bpR[m] = 0.0; }
-    if (lim && a.trans > 0) {
-        const bool cor = a.order == 2 && a.trans == 2;
-        double A[MEQN], Pf[MEQN];
+    for (int m = 0; m < MEQN; m++) { cqxx[m] = 0.0; bmL[m] = 0.0; bpL[m] = 0.0; bmR[m] = 0.0; bpR[m] = 0.0; }
+    if (!flat) {                                   // a line of one state carries no waves
+        if (a.order == 2) {
+            double dr[MW], dl[MW];
+            if (a.limit_any) {
+                double alr[MW], roer[NR];
 #pragma unroll
-        for (int m = 0; m < MEQN; m++) {
-            A[m] = cor ? amdq[m] + cqxx[m] : amdq[m];
-            Pf[m] = cor ? apdq[m] - cqxx[m] : apdq[m];
+                for (int p = 0; p < MW; p++) alr[p] = ctx.shfl_down(al[p]);
+#pragma unroll
+                for (int r = 0; r < NR; r++) roer[r] = r < RP::NROE_WAVE ? ctx.shfl_down(roe[r]) : 0.0;
+                dense_dots<D, IXY>(al, roe, alr, roer, dr);
+#pragma unroll
+                for (int p = 0; p < MW; p++) dl[p] = ctx.shfl_up(dr[p]);
+            }
+            dense_correct<D, IXY>(a, al, roe, dr, dl, dtn, lim, cqxx);
         }
-        const double noaux[1] = {0.0};
-        // a zero fluctuation splits into zeros (up to the sign of zero), so
-        // its transverse solve is skipped
-        bool nzA = false, nzP = false;
+        // ---------------- transverse splits ----------------
+        if (a.trans > 0) {
+            const bool cor = a.order == 2 && a.trans == 2;
+            double A[MEQN], Pf[MEQN];
 #pragma unroll
-        for (int m = 0; m < MEQN; m++) { nzA = nzA || A[m] != 0.0; nzP = nzP || Pf[m] != 0.0; }
-        if (nzA) RP::template rpt2<IXY>(1, A, roe, noaux, noaux, noaux, a.prm, bmL, bpL);
-        if (nzP) RP::template rpt2<IXY>(2, Pf, roe, noaux, noaux, noaux, a.prm, bmR, bpR);
+            for (int m = 0; m < MEQN; m++) {
+                A[m] = cor ? amdq[m] + cqxx[m] : amdq[m];
+                Pf[m] = cor ? apdq[m] - cqxx[m] : apdq[m];
+            }
+            const bool sub = __all_sync(0xffffffffu, D::subsonic(roe) || !lim);
+            dense_split<D, IXY>(A, roe, sub, lim, bmL, bpL);
+            dense_split<D, IXY>(Pf, roe, sub, lim, bmR, bpR);
+        }
     }
+#pragma unroll
+    for (int m = 0; m < MEQN; m++) fadd[m] = 0.5 * cqxx[m];
 
     // ---------------- the slice's contributions to cell k ----------------
     // what interface k+1 hands to its left cell (this lane's cell k)
@@ -211,10 +183,10 @@ CLAW2_HD void lean_chunk(const StepArgs& a, Ctx& ctx, const double* H, double* Q
         const double hr = 0.5 * dtn;
 #pragma unroll
         for (int m = 0; m < MEQN; m++) {
-            const double qadd = (0.0 - dtn * apdq[m]) - y0[m];
+            const double qadd = -(dtn * apdq[m]) - y0[m];
             const double dF = y1[m] - fadd[m];
-            const double g1 = (0.0 - y2[m]) - hr * bmR[m];
-            const double g2 = (0.0 - y3[m]) - hr * bpR[m];
+            const double g1 = -y2[m] - hr * bmR[m];
+            const double g2 = -y3[m] - hr * bpR[m];
             C0[m] = dtt * g2;
             C1[m] = qadd;
             C2[m] = dtn * dF;
