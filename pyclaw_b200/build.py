@@ -3,8 +3,8 @@
     python -m pyclaw_b200.build          # or pyclaw_b200.build.build()
 
 Compiles the sources under csrc/ (claw2_capi.cu: the plain step and the C ABI;
-claw2_acoustics.cu: the unsplit acoustics step; claw2_batch.cu: the batched
-form; claw2_adjoint.cu: multi-shot acoustics and its adjoint) with nvcc for
+claw2_acoustics.cu: the unsplit acoustics step; claw2_lean.cu: the Euler and
+shallow-water step; claw2_batch.cu: the batched form; claw2_adjoint.cu: multi-shot acoustics and its adjoint) with nvcc for
 sm_100a only, without FMA contraction so that the step keeps the reference's
 rounding, as objects compiled in parallel under pyclaw_b200/_build/, and links
 them into pyclaw_b200/libclaw2.so (in-tree, so the library travels with the
@@ -21,6 +21,7 @@ LIB = os.path.join(HERE, "libclaw2.so")
 SRCS = [os.path.join(HERE, "csrc", "claw2_capi.cu"),
         os.path.join(HERE, "csrc", "claw2_batch.cu"),
         os.path.join(HERE, "csrc", "claw2_acoustics.cu"),
+        os.path.join(HERE, "csrc", "claw2_lean.cu"),
         os.path.join(HERE, "csrc", "claw2_adjoint.cu")]
 OBJDIR = os.path.join(HERE, "_build")
 DEPS = SRCS + [os.path.join(HERE, "csrc", "claw2_kernels.cuh"),

@@ -2,8 +2,6 @@
 //
 // Built for sm_100a with --fmad=false (no FMA contraction, so the step
 // reproduces the reference's operation-by-operation rounding).
-#include <cuda.h>
-#include <cudaTypedefs.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -20,7 +18,6 @@
 #include "claw2_host.h"
 #include "claw2_kernels.cuh"
 #include "claw2_launch.cuh"
-#include "claw2_lean.cuh"
 
 namespace claw2 {
 
@@ -35,39 +32,6 @@ __global__ void __launch_bounds__(NT, CLAW2_MINB) step_kernel(StepArgs a)
     extern __shared__ double smem_dyn[];
     DevCtx ctx{smem_dyn};
     step_tile<RP, TX, TY, NT, SPLIT>(a, ctx);
-}
-
-// The dense-wave solvers without aux arrays (Euler, shallow water) have the
-// same data movement in a lean unsplit body (claw2_lean.cuh): shuffles
-// instead of shared-memory exchange, one block barrier per chunk.
-template <class RP> struct HasLean { static constexpr bool value = false; };
-template <> struct HasLean<RpEuler<false>> { static constexpr bool value = true; };
-template <> struct HasLean<RpEuler<true>> { static constexpr bool value = true; };
-template <> struct HasLean<RpShallow> { static constexpr bool value = true; };
-
-// lean tiles: 28 x 28 cells, so that a line's 32 lanes hold its 32 cells.
-// Two block sizes, one line of a chunk per warp: 512 threads (one CTA per SM,
-// 16 lines per chunk) halve a tile's latency, which decides the step when the
-// grid has few tiles per SM (a launch of a few waves ends with a partial
-// one); 256 threads (two CTAs per SM) let one CTA's waits (its halo copy, its
-// barriers, the launch of the next CTA) overlap the other's work, which
-// decides it when the grid has many tiles, most of them cheap.
-constexpr int LTX = 28, LTY = 28;
-constexpr int LEAN_BIG_BLOCK_TILES = 8 * 148;   // grids of at most 8 tiles per SM of a B200 use 512 threads
-
-// tm0 / tm1: tensor maps of the input state (see lean_tile_at), passed as
-// __grid_constant__ parameters so the TMA unit can read them in place.
-template <class RP, int NT>
-__global__ void __launch_bounds__(NT, 512 / NT)
-lean_step_kernel(StepArgs a, const __grid_constant__ CUtensorMap tm0, const __grid_constant__ CUtensorMap tm1)
-{
-    extern __shared__ double smem_dyn[];
-    __shared__ __align__(8) uint64_t halo_bar;
-    chain_wait();
-    DevCtx ctx{smem_dyn};
-    const TileId t{(int)blockIdx.x, (int)blockIdx.y, (int)gridDim.x, (int)gridDim.y,
-                   (int)(blockIdx.y * gridDim.x + blockIdx.x), (int)(gridDim.x * gridDim.y)};
-    lean_tile_at<RP, LTX, LTY, NT>(a, ctx, t, &tm0, &tm1, &halo_bar);
 }
 
 // Tile shapes: a line of a chunk has 32 interface slots, so TX+3, TY+3 <= 32.
@@ -263,11 +227,11 @@ bool march_body(const claw2_problem* p)
            (p->rp == CLAW2_RP_ACOUSTICS || p->rp == CLAW2_RP_VC_ACOUSTICS);
 }
 
-// Problems stepped by the lean body (launch_step_t): unsplit Euler and
-// shallow water without capacity or f-waves.
+// Problems stepped by the lean body (launch_step): Euler and shallow water
+// without capacity or f-waves.
 bool lean_body(const claw2_problem* p)
 {
-    return p->transverse >= 0 && p->index_capa < 0 && !p->use_fwave &&
+    return p->index_capa < 0 && !p->use_fwave &&
            (p->rp == CLAW2_RP_EULER_4WAVE || p->rp == CLAW2_RP_EULER_5WAVE || p->rp == CLAW2_RP_SHALLOW_ROE);
 }
 
@@ -285,8 +249,8 @@ void tiles(const claw2_problem* p, int* nbx, int* nby)
     int tx = split ? STX : UTX, ty = split ? STY : UTY;
     // the marching body counts in tiles only for the scratch it is given
     if (march_body(p) && march_small_grid(p->mx, p->my)) tx = ty = MARCH_SMALL_TILE;
-    // the lean body's tiles (launch_step_t)
-    if (lean_body(p)) { tx = LTX; ty = LTY; }
+    // as does the lean body
+    if (lean_body(p)) tx = ty = LEAN_T;
     *nbx = (p->mx + tx - 1) / tx;
     *nby = (p->my + ty - 1) / ty;
 }
@@ -307,75 +271,12 @@ void set_scratch(void* scratch, StepArgs& a)
     a.partials = reinterpret_cast<double*>(static_cast<char*>(scratch) + 64);
 }
 
-// cuTensorMapEncodeTiled from the driver, found through the runtime (no link
-// against libcuda, so the library still loads on a machine without a GPU)
-PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder()
-{
-    static std::atomic<void*> fn{nullptr};
-    void* f = fn.load(std::memory_order_acquire);
-    if (!f) {
-        cudaDriverEntryPointQueryResult q = cudaDriverEntryPointSymbolNotFound;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &f, cudaEnableDefault, &q) != cudaSuccess ||
-            q != cudaDriverEntryPointSuccess || !f)
-            return nullptr;
-        fn.store(f, std::memory_order_release);
-    }
-    return reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(f);
-}
-
-// Tensor map of one state buffer for the lean body's halo boxes: the ghosted
-// planes (mx+4 columns, my+4 rows, meqn fields; rows ld doubles apart, planes
-// `plane` doubles apart), boxes of 16 x 32 x meqn, 128-byte swizzle, zeros
-// outside the ghosted array.
-int halo_tensor_map(CUtensorMap* m, const double* q, const StepArgs& a, int meqn)
-{
-    auto encode = tensor_map_encoder();
-    if (!encode) return CLAW2_ERR_CUDA;
-    if ((reinterpret_cast<uintptr_t>(q) & 15u) != 0) return CLAW2_ERR_INVALID;
-    const cuuint64_t dims[3] = {(cuuint64_t)(a.mx + 2 * CLAW2_NUM_GHOST), (cuuint64_t)(a.my + 2 * CLAW2_NUM_GHOST),
-                                (cuuint64_t)meqn};
-    const cuuint64_t strides[2] = {(cuuint64_t)a.ld * sizeof(double), (cuuint64_t)a.plane * sizeof(double)};
-    const cuuint32_t box[3] = {16, 32, (cuuint32_t)meqn};
-    const cuuint32_t estr[3] = {1, 1, 1};
-    const CUresult r = encode(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 3, const_cast<double*>(q), dims, strides, box, estr,
-                              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                              CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    return r == CUDA_SUCCESS ? CLAW2_OK : CLAW2_ERR_CUDA;
-}
-
 // bytes of halo that lean-body CTAs wait for in vain (claw2_debug_halo_shortfall)
 std::atomic<int> g_halo_shortfall{0};
-
-// chained: the previous operation in the stream is a step kernel of the same
-// device loop (launch_kernel).
-template <class RP, int NT>
-int launch_lean_t(const StepArgs& a0, int nbx, int nby, cudaStream_t st, bool chained)
-{
-    StepArgs a = a0;
-    a.halo_shortfall = g_halo_shortfall.load(std::memory_order_relaxed);
-    using SM = LeanSmem<RP, LTX, LTY, NT>;
-    auto kern = lean_step_kernel<RP, NT>;
-    static std::atomic<uint64_t> optin{0};
-    if (smem_optin(optin, kern, SM::bytes) != cudaSuccess) return CLAW2_ERR_CUDA;
-    CUtensorMap tm0, tm1;
-    int rc = halo_tensor_map(&tm0, a.ctrl ? a.q0 : a.qin, a, RP::MEQN);
-    if (!rc) rc = a.ctrl ? halo_tensor_map(&tm1, a.q1, a, RP::MEQN) : (tm1 = tm0, CLAW2_OK);
-    if (rc) return rc;
-    return launch_kernel(kern, dim3(nbx, nby), NT, SM::bytes, st, chained, a, tm0, tm1);
-}
-
-template <class RP>
-int launch_lean(const StepArgs& a, int nbx, int nby, cudaStream_t st, bool chained)
-{
-    if ((long long)nbx * nby <= LEAN_BIG_BLOCK_TILES) return launch_lean_t<RP, 512>(a, nbx, nby, st, chained);
-    return launch_lean_t<RP, 256>(a, nbx, nby, st, chained);
-}
 
 template <class RP, bool SPLIT>
 int launch_step_t(const StepArgs& a, int nbx, int nby, cudaStream_t st, bool chained)
 {
-    if constexpr (!SPLIT && HasLean<RP>::value)
-        if (a.capa < 0 && !a.fwave) return launch_lean<RP>(a, nbx, nby, st, chained);
     constexpr int TX = SPLIT ? STX : UTX, TY = SPLIT ? STY : UTY, NT = SPLIT ? SNT : UNT;
     using SM = TileSmem<RP, TX, TY, NT, SPLIT>;
     auto kern = step_kernel<RP, TX, TY, NT, SPLIT>;
@@ -389,9 +290,18 @@ int launch_step_t(const StepArgs& a, int nbx, int nby, cudaStream_t st, bool cha
 int launch_step(const claw2_problem* p, const StepArgs& a, cudaStream_t st, bool chained = false)
 {
     if (march_body(p)) return launch_march(p->rp, a, st, chained);
+    const bool split = p->transverse < 0;
+    // the lean body's halo copies start on 16-byte boundaries; other buffers keep
+    // the general split body (unsplit they are refused)
+    const uintptr_t start = a.ctrl ? reinterpret_cast<uintptr_t>(a.q0) | reinterpret_cast<uintptr_t>(a.q1)
+                                   : reinterpret_cast<uintptr_t>(a.qin);
+    if (lean_body(p) && (!split || (start & 15u) == 0)) {
+        StepArgs l = a;
+        l.halo_shortfall = g_halo_shortfall.load(std::memory_order_relaxed);
+        return launch_lean(p->rp, split, l, st, chained);
+    }
     int nbx, nby;
     tiles(p, &nbx, &nby);
-    const bool split = p->transverse < 0;
     switch (p->rp) {
     case CLAW2_RP_ACOUSTICS:
         return split ? launch_step_t<RpAcoustics, true>(a, nbx, nby, st, chained) : launch_step_t<RpAcoustics, false>(a, nbx, nby, st, chained);

@@ -679,13 +679,11 @@ CLAW2_HD void euler_radial_source(double (&v)[MEQN], double rad, double gamma1, 
     }
 }
 
-// QP: row pitch of Qx in doubles (TX unless the body pads its rows).
-// fault: the tile could not be computed (its input never arrived): nothing is
-// written and the step reports CLAW2_ERR_TIMEOUT (controlled mode) or a NaN
-// CFL number.
+// Write a tile's final values and the ghost cells that are images of them;
+// whether this thread saw one that is not finite.  QP: row pitch of Qx in doubles
+// (TX unless the body pads its rows).
 template <int MEQN, int TX, int TY, int NT, int QP = TX, class Ctx>
-CLAW2_HD void finish_tile(const StepArgs& a, Ctx& ctx, const TileId& tile, const double* Qx, int QSTR, double* red,
-                          double* qout, int i0, int j0, double cflm, double dt, bool fault = false)
+CLAW2_HD bool store_tile(const StepArgs& a, Ctx& ctx, const double* Qx, int QSTR, double* qout, int i0, int j0, double dt)
 {
     const int tid = ctx.tid();
     int bad = 0;
@@ -699,37 +697,45 @@ CLAW2_HD void finish_tile(const StepArgs& a, Ctx& ctx, const TileId& tile, const
         if (a.src == CLAW2_SRC_EULER_RADIAL)
             euler_radial_source<MEQN>(v, a.aux[qoff(a, a.src_aux, i, j)], a.prm[1], dt);
     };
-    if (!fault) {
 #pragma unroll
-        for (int k = 0; k < NIT; k++) {
-            const int idx = tid + k * NT;
-            const int ci = idx % TX, cj = idx / TX;
-            const int i = i0 + ci, j = j0 + cj;
-            if (idx < TX * TY && i < a.mx && j < a.my) {
-                double v[MEQN];
-                cell_value(ci, cj, i, j, v);
+    for (int k = 0; k < NIT; k++) {
+        const int idx = tid + k * NT;
+        const int ci = idx % TX, cj = idx / TX;
+        const int i = i0 + ci, j = j0 + cj;
+        if (idx < TX * TY && i < a.mx && j < a.my) {
+            double v[MEQN];
+            cell_value(ci, cj, i, j, v);
 #pragma unroll
-                for (int m = 0; m < MEQN; m++) {
-                    if (!isfinite(v[m])) bad = 1;
-                    qout[qoff(a, m, i, j)] = v[m];
-                }
-            }
-        }
-        const bool edge = i0 <= 1 || i0 + TX >= a.mx - 2 || j0 <= 1 || j0 + TY >= a.my - 2;
-        if (a.ghost_fused && edge) {
-            for (int idx = tid; idx < TX * TY; idx += NT) {
-                const int ci = idx % TX, cj = idx / TX;
-                const int i = i0 + ci, j = j0 + cj;
-                if (i >= a.mx || j >= a.my) continue;
-                if (i > 1 && i < a.mx - 2 && j > 1 && j < a.my - 2) continue;   // no images
-                double v[MEQN];
-                cell_value(ci, cj, i, j, v);
-                write_ghosts<MEQN>(a, qout, i, j, v);
+            for (int m = 0; m < MEQN; m++) {
+                if (!isfinite(v[m])) bad = 1;
+                qout[qoff(a, m, i, j)] = v[m];
             }
         }
     }
+    const bool edge = i0 <= 1 || i0 + TX >= a.mx - 2 || j0 <= 1 || j0 + TY >= a.my - 2;
+    if (a.ghost_fused && edge) {
+        for (int idx = tid; idx < TX * TY; idx += NT) {
+            const int ci = idx % TX, cj = idx / TX;
+            const int i = i0 + ci, j = j0 + cj;
+            if (i >= a.mx || j >= a.my) continue;
+            if (i > 1 && i < a.mx - 2 && j > 1 && j < a.my - 2) continue;   // no images
+            double v[MEQN];
+            cell_value(ci, cj, i, j, v);
+            write_ghosts<MEQN>(a, qout, i, j, v);
+        }
+    }
+    return bad != 0;
+}
 
-    report_cfl<NT>(a, ctx, tile, red, cflm, bad != 0, fault);
+// fault: the tile could not be computed (its input never arrived): nothing is
+// written and the step reports CLAW2_ERR_TIMEOUT (controlled mode) or a NaN
+// CFL number.
+template <int MEQN, int TX, int TY, int NT, int QP = TX, class Ctx>
+CLAW2_HD void finish_tile(const StepArgs& a, Ctx& ctx, const TileId& tile, const double* Qx, int QSTR, double* red,
+                          double* qout, int i0, int j0, double cflm, double dt, bool fault = false)
+{
+    const bool bad = !fault && store_tile<MEQN, TX, TY, NT, QP>(a, ctx, Qx, QSTR, qout, i0, j0, dt);
+    report_cfl<NT>(a, ctx, tile, red, cflm, bad, fault);
 }
 
 // f(IntC<0>{}), ..., f(IntC<N-1>{}): a loop whose index is a compile-time constant
@@ -911,6 +917,39 @@ struct DevCtx {
     __device__ __forceinline__ bool warp_any(bool p) const { return __any_sync(0xffffffffu, p) != 0; }
     __device__ __forceinline__ void prefetch_l2(const void* p) const { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 };
+
+// A CTA's CFL maximum (one thread), and in the last CTA to arrive the step's:
+// CFL numbers are >= 0, so their bits order as integers and one atomic maximum
+// per CTA collects them in the cell that a.partials points to (zero between
+// launches); a non-finite state counts as infinity, a tile that could not be
+// computed as more.  No scratch grows with the tiles.
+__device__ __forceinline__ void collect_cfl(const StepArgs& a, DevCtx& ctx, int ntiles, double cfl, bool nonfinite, bool fault)
+{
+    unsigned long long* cell = reinterpret_cast<unsigned long long*>(a.partials);
+    constexpr unsigned long long inf = 0x7ff0000000000000ULL, lost = 0x7ff8000000000000ULL;
+    atomicMax(cell, fault ? lost : nonfinite ? inf : (unsigned long long)__double_as_longlong(cfl));
+    __threadfence();
+    if (atomicAdd(a.ticket, 1u) != (unsigned)(ntiles - 1)) return;
+    __threadfence();
+    const unsigned long long top = atomicExch(cell, 0ULL);
+    *a.ticket = 0u;
+    finish_step(a, ctx, top >= inf ? 0.0 : __longlong_as_double((long long)top), top >= lost ? 2 : top >= inf ? 1 : 0);
+    __threadfence();
+}
+
+// the same for a CTA of NT threads.  red: NT/32 doubles of shared memory.
+template <int NT>
+__device__ __forceinline__ void report_cell(const StepArgs& a, DevCtx& ctx, int ntiles, double* red, double cflm, bool bad,
+                                            bool fault)
+{
+    const double mw = ctx.warp_max(cflm);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = mw;
+    const bool nf = __syncthreads_or(bad || cflm != cflm);
+    if (threadIdx.x != 0) return;
+    double cfl = 0.0;
+    for (int w = 0; w < NT / 32; w++) cfl = cfl > red[w] ? cfl : red[w];
+    collect_cfl(a, ctx, ntiles, cfl, nf, fault);
+}
 #endif
 
 }  // namespace claw2

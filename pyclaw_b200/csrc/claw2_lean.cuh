@@ -1,15 +1,17 @@
-// claw2_lean.cuh -- a leaner unsplit tile body for the solvers with dense
-// waves and no aux arrays (Euler 4- and 5-wave Roe, shallow-water Roe).
+// claw2_lean.cuh -- the step of the solvers with dense waves and no aux arrays
+// (Euler 4- and 5-wave Roe, shallow-water Roe), unsplit or split, on square
+// tiles of T = 28 or 12 cells.
 //
-// Same step as step_tile_at (step2.f90:92-248 / flux2.f90:104-206) with the
-// same operations in the same order, so the results are the same values; only
-// the data movement differs, as in the acoustics body of claw2_light.cuh:
-//  - each lane computes the quantities of one cell that the normal solve
-//    needs (dense_cell: square roots, pressures, Roe-average numerators) and
-//    takes those of the cell right of its interface from the next lane, so
-//    each cell's are computed once per line instead of once per interface;
-//    with TX = 28 the 32 lanes hold the 32 cells i0-2 .. i0+29 of the line's
-//    31 interfaces;
+// Same step as step_tile_at (step2.f90:92-248, step2ds.f90:96-252, flux2.f90:
+// 104-206) with the same operations in the same order, so the results are the
+// same values; only the data movement differs:
+//  - a line of the tile (a row in the x sweep, a column in the y sweep) is held
+//    by T + 4 lanes, one cell each, cells i0-2 .. i0+T+1: a warp holds one line
+//    of a 28-tile or two of a 12-tile;
+//  - each lane computes the quantities of its cell that the normal solve needs
+//    (dense_cell: square roots, pressures, Roe-average numerators) and takes
+//    those of the cell right of its interface from the next lane, so each
+//    cell's are computed once per line instead of once per interface;
 //  - the solves are those of claw2_dense.cuh: the same bits from fewer
 //    instructions and no divergent divisions;
 //  - the normal solve stays in registers; for the limiter each lane takes its
@@ -21,12 +23,15 @@
 //    splits are passed over;
 //  - what the cell left of an interface needs from it (dtdx*amdq, fadd and
 //    the two transverse splits) moves one lane by shuffle;
-//  - a cell's own-line contributions stay in registers; only the two
+//  - unsplit, a cell's own-line contributions stay in registers; only the two
 //    cross-line terms (to the line above and below) go through a
 //    double-buffered shared array: one block barrier per chunk of lines;
-//  - the tile's whole input halo (rows j0-2..j0+TY+1, columns i0-2..i0+TX+1)
-//    is staged in shared memory once by the tensor memory accelerator (two
-//    boxes of 16 columns x 32 rows x MEQN fields, 128-byte swizzle; see
+//  - split, a line depends on no other: the x sweep rewrites the rows of the
+//    staged halo in place, and one block barrier later the y sweep reads its
+//    columns;
+//  - the tile's whole input halo (rows j0-2..j0+T+1, columns i0-2..i0+T+1)
+//    is staged in shared memory once by the tensor memory accelerator (boxes
+//    of 16 columns x T+4 rows x MEQN fields, 128-byte swizzle; see
 //    claw2_tma.cuh) while the threads wait on an mbarrier; x lines read rows
 //    of it and y lines read down its columns;
 //  - a tile whose staged halo holds one state skips both sweeps: every
@@ -36,9 +41,16 @@
 // Bound by the latency of the FP64 chains and by issue: 128 registers a thread
 // leave 4 warps per SM quarter, which issue 44% of the cycles (FP64 pipe 36%
 // busy; stalled on dependences 2.1 and barriers 1.4 of the 8 warp-cycles per
-// instruction).  Euler 4-wave, us a step on a B200: 1280 x 320 66.8 (75.4 with
-// the solves of claw2_riemann.cuh), 1500^2 283 (331), 256^2 29.9 (36.7); 5-wave
-// 1500^2 453 (532); shallow water 1500^2 292 (367), 256^2 22.5 (26.4).
+// instruction).  80 registers and 6 warps spill and lose (Euler 1500^2 391 us
+// against 280, split 197 against 175).  us a step on a B200, before (the solves
+// of claw2_riemann.cuh; split, the general body; 28-tiles only) and now:
+//                     64 x 48      256^2        641 x 163    1500^2
+//   Euler 4 unsplit   36.5  15.3   36.7  29.4   36.8  30.4   331  280
+//   Euler 4 split     44.5  12.3   47.9  23.2   49.9  23.3   394  175
+//   Euler 5 unsplit   40.0  17.0   40.0  34.1   40.0  34.5   532  368
+//   Euler 5 split     47.8  13.9   48.9  25.4   49.2  25.6   697  214
+//   shallow unsplit   25.8  12.2   26.4  21.1   26.6  22.3   367  282
+//   shallow split     29.5  10.2   31.5  16.3   32.7  18.4   275  184
 #pragma once
 
 #include "claw2_dense.cuh"
@@ -47,23 +59,26 @@
 
 namespace claw2 {
 
-// Shared memory of the lean body (doubles): the staged input halo (2 boxes x
-// MEQN fields x TR rows x 16 columns, at a 1024-byte boundary for the
-// swizzle), the tile state, the cross-line exchange (2 buffers x 2 terms x
-// MEQN x NT) and the reduction scratch; `bytes` includes up to 1 KB of
-// alignment padding in front of the halo.
-template <class RP, int TX, int TY, int NT> struct LeanSmem {
+// Shared memory of the lean body (doubles): the staged input halo (T+4 rows and
+// columns, in boxes of 16 columns, at a 1024-byte boundary for the swizzle), the
+// tile's new state, unsplit the cross-line exchange (2 buffers x 2 terms x MEQN x
+// cells of a chunk), and the reduction scratch; `bytes` includes up to 1 KB of alignment
+// padding in front of the halo.
+template <class RP, int T, int NT, bool SPLIT> struct LeanSmem {
     static constexpr int MEQN = RP::MEQN;
-    static constexpr int QP = TX | 1;            // row pitch of the tile state: odd, so that
+    static constexpr int QP = T | 1;             // row pitch of the tile state: odd, so that
                                                  // y lines walking down a column avoid bank conflicts
-    static constexpr int QX = MEQN * TY * QP;
-    static constexpr int CX = 2 * 2 * MEQN * NT;
-    static constexpr int TR = TY + 4;            // rows j0-2 .. j0+TY+1
+    static constexpr int QX = MEQN * T * QP;
+    static constexpr int LPC = NT / (T + 4);      // lines of a chunk
+    static constexpr int NX = LPC * T;           // their cells
+    static constexpr int CX = SPLIT ? 0 : 2 * 2 * MEQN * NX;
+    static constexpr int TR = T + 4;             // rows j0-2 .. j0+T+1; also the lanes of a line
+    static constexpr int NBOX = TR / 16;
     static constexpr int BOX = MEQN * TR * 16;   // one box: columns 16b .. 16b+15 of the halo
-    static constexpr int HS = 2 * BOX;
-    static constexpr int total = HS + QX + CX + NT;
+    static constexpr int HS = NBOX * BOX;
+    static constexpr int total = HS + QX + CX + NT / 32;
     static constexpr int bytes = total * 8 + 1024;
-    static_assert(TX + 4 == 32 && TR == 32, "the halo is two 16 x 32 boxes");
+    static_assert(TR == 16 || TR == 32, "lines of 16 or 32 lanes, boxes of 16 columns");
     static_assert((BOX * 8) % 1024 == 0, "each box starts on a 1024-byte boundary");
 };
 
@@ -74,87 +89,134 @@ __device__ __forceinline__ int lean_hidx(int m, int r, int c)
     return (c >> 4) * (MEQN * TR * 16) + m * (TR * 16) + swz128(r, c & 15);
 }
 
+// The part of a line that both forms of the step share.  `line` is a line of the
+// halo, the lane's interface is k, its left cell k-1.
+template <class RP, int IXY, int T> struct LeanLine {
+    using D = typename DenseOf<RP>::type;
+    static constexpr int MEQN = RP::MEQN, MW = RP::MW, TR = T + 4, NSLOT = T + 3;
+    int slot, k, len;
+    bool ifok, lim;              // a limiter neighbour; an interface whose flux counts
+    bool flat;                   // the warp's lines carry no waves
+    double q[MEQN];              // cell k
+    double amdq[MEQN], apdq[MEQN], roe[D::NR], cqxx[MEQN];
+
+    // the staged input of cell (kk along the line, ll across it)
+    static __device__ __forceinline__ int at(int m, int kk, int ll, int i0, int j0)
+    {
+        return IXY == 1 ? lean_hidx<MEQN, TR>(m, ll - j0 + 2, kk - i0 + 2) : lean_hidx<MEQN, TR>(m, kk - j0 + 2, ll - i0 + 2);
+    }
+    // normal solve, CFL number, second-order correction
+    template <class Ctx>
+    __device__ __forceinline__ void solve(const StepArgs& a, Ctx& ctx, const double* H, int i0, int j0, int line, bool lineok,
+                                          double dtn, double& cflm)
+    {
+        constexpr int NR = D::NR, NCD = D::NCD;
+        slot = ctx.tid() & (TR - 1);
+        len = IXY == 1 ? a.mx : a.my;
+        k = (IXY == 1 ? i0 : j0) - 1 + slot;
+        ifok = lineok && slot < NSLOT && k <= len + 1;
+        lim = ifok && slot >= 1 && slot <= NSLOT - 2 && k >= 0 && k <= len;
+        double al[MW];
+        {
+            // this lane's cell k-1, and cell k from the next lane
+            double qL[MEQN], L[NCD], R[NCD];
+#pragma unroll
+            for (int m = 0; m < MEQN; m++) {
+                qL[m] = H[at(m, k - 1, line, i0, j0)];
+                q[m] = H[at(m, slot < NSLOT ? k : k - 1, line, i0, j0)];
+            }
+            dense_cell<D, IXY>(a, qL, lineok && k - 1 <= len + 1, L);
+#pragma unroll
+            for (int f = 0; f < NCD; f++) R[f] = f != D::S0 ? ctx.shfl_down(L[f]) : 0.0;
+            bool eq = true;
+#pragma unroll
+            for (int m = 0; m < MEQN; m++) eq = eq && qL[m] == q[m];
+            flat = __all_sync(0xffffffffu, eq || !ifok);
+            dense_normal<D, IXY>(a, qL, q, L, R, ifok, al, amdq, apdq, roe);
+        }
+        if (lim) {
+            const double c = fabs(dtn) * D::top_speed(roe);     // the largest of dtn s and -dtn s over the waves
+            cflm = cflm > c ? cflm : c;
+        }
+#pragma unroll
+        for (int m = 0; m < MEQN; m++) cqxx[m] = 0.0;
+        if (flat || a.order != 2) return;
+        double dr[MW], dl[MW];
+        if (a.limit_any) {
+            double alr[MW], roer[NR];
+#pragma unroll
+            for (int p = 0; p < MW; p++) alr[p] = ctx.shfl_down(al[p]);
+#pragma unroll
+            for (int r = 0; r < NR; r++) roer[r] = r < RP::NROE_WAVE ? ctx.shfl_down(roe[r]) : 0.0;
+            dense_dots<D, IXY>(al, roe, alr, roer, dr);
+#pragma unroll
+            for (int p = 0; p < MW; p++) dl[p] = ctx.shfl_up(dr[p]);
+        }
+        dense_correct<D, IXY>(a, al, roe, dr, dl, dtn, lim, cqxx);
+    }
+};
+
+// One line of the split step (step2ds.f90:96-252): the x sweep rewrites its row of
+// H, the y sweep writes its column of the new state; `own`: the line's cells are
+// swept (ghost columns only count in the CFL number).
+template <class RP, int IXY, int T, int NT, class Ctx>
+__device__ __forceinline__ void lean_split_line(const StepArgs& a, Ctx& ctx, double* H, double* Qx, int i0, int j0, int line,
+                                                bool lineok, bool own, double dtn, double& cflm)
+{
+    using LL = LeanLine<RP, IXY, T>;
+    using SM = LeanSmem<RP, T, NT, true>;
+    constexpr int MEQN = RP::MEQN;
+    LL S;
+    S.solve(a, ctx, H, i0, j0, line, lineok, dtn, cflm);
+    double v[MEQN];
+#pragma unroll
+    for (int m = 0; m < MEQN; m++) {
+        const double y0 = ctx.shfl_down(dtn * S.amdq[m]), y1 = ctx.shfl_down(0.5 * S.cqxx[m]);
+        v[m] = S.q[m] + (-(dtn * S.apdq[m]) - y0) - dtn * (y1 - 0.5 * S.cqxx[m]);
+    }
+    __syncwarp();                                  // the row has been read
+    if (own && S.lim && S.slot <= T && S.k < S.len) {
+#pragma unroll
+        for (int m = 0; m < MEQN; m++) {
+            if (IXY == 1) H[LL::at(m, S.k, line, i0, j0)] = v[m];
+            else Qx[(m * T + (S.k - j0)) * SM::QP + (line - i0)] = v[m];
+        }
+    }
+}
+
 // One chunk of one sweep direction (arguments as in sweep_chunk); CXb is the
 // half of the exchange array this chunk uses.
-template <class RP, int IXY, int TX, int TY, int NT, class Ctx>
+template <class RP, int IXY, int T, int NT, class Ctx>
 __device__ __forceinline__ void lean_chunk(const StepArgs& a, Ctx& ctx, const double* H, double* Qx, double* CXb, int i0, int j0,
                          int line, int cfirst, int clast, bool lineok, double dtn, double dtt, double& cflm)
 {
-    constexpr int MEQN = RP::MEQN, MW = RP::MW;
-    using SM = LeanSmem<RP, TX, TY, NT>;
-    constexpr int TR = SM::TR;
-    // the staged input of cell (kk along the slice, ll across it)
-    auto hq = [&](int m, int kk, int ll) -> double {
-        return IXY == 1 ? H[lean_hidx<MEQN, TR>(m, ll - j0 + 2, kk - i0 + 2)]
-                        : H[lean_hidx<MEQN, TR>(m, kk - j0 + 2, ll - i0 + 2)];
-    };
-    constexpr int NCELL = IXY == 1 ? TX : TY;
-    constexpr int NSLOT = NCELL + 3;
-    const int tid = ctx.tid();
-    const int slot = tid & 31;
-    const int len = IXY == 1 ? a.mx : a.my;
-    const int k = (IXY == 1 ? i0 : j0) - 1 + slot;
-    const bool ifok = lineok && slot < NSLOT && k <= len + 1;
-    const bool lim = ifok && slot >= 1 && slot <= NSLOT - 2 && k >= 0 && k <= len;
+    constexpr int MEQN = RP::MEQN;
+    using SM = LeanSmem<RP, T, NT, false>;
+    using LL = LeanLine<RP, IXY, T>;
+    using D = typename LL::D;
+    constexpr int NCELL = T, LANES = SM::TR;
+    LL S;
+    S.solve(a, ctx, H, i0, j0, line, lineok, dtn, cflm);
+    const int tid = ctx.tid(), slot = S.slot, k = S.k, len = S.len;
+    const bool lim = S.lim;
+    const double (&amdq)[MEQN] = S.amdq, (&apdq)[MEQN] = S.apdq, (&cqxx)[MEQN] = S.cqxx;
+    auto hq = [&](int m, int kk, int ll) -> double { return H[LL::at(m, kk, ll, i0, j0)]; };
 
-    using D = typename DenseOf<RP>::type;
-    constexpr int NR = D::NR, NCD = D::NCD;
-    // interfaces whose fluxes and waves count, and whether this lane's is one
-    // (lim) or a limiter neighbour (ifok)
-    double al[MW], amdq[MEQN], apdq[MEQN], roe[NR], cqxx[MEQN], fadd[MEQN];
-    bool flat;
-    {
-        // this lane's cell k-1, and cell k from the next lane
-        double qL[MEQN], qR[MEQN], L[NCD], R[NCD];
-        const bool cellok = lineok && k - 1 <= len + 1;
+    double fadd[MEQN], bmL[MEQN], bpL[MEQN], bmR[MEQN], bpR[MEQN];
 #pragma unroll
-        for (int m = 0; m < MEQN; m++) { qL[m] = hq(m, k - 1, line); qR[m] = hq(m, slot < 31 ? k : k - 1, line); }
-        dense_cell<D, IXY>(a, qL, cellok, L);
+    for (int m = 0; m < MEQN; m++) { bmL[m] = 0.0; bpL[m] = 0.0; bmR[m] = 0.0; bpR[m] = 0.0; }
+    // ---------------- transverse splits (a line of one state carries no waves) ----------------
+    if (!S.flat && a.trans > 0) {
+        const bool cor = a.order == 2 && a.trans == 2;
+        double A[MEQN], Pf[MEQN];
 #pragma unroll
-        for (int f = 0; f < NCD; f++) R[f] = f != D::S0 ? ctx.shfl_down(L[f]) : 0.0;
-        bool eq = true;
-#pragma unroll
-        for (int m = 0; m < MEQN; m++) eq = eq && qL[m] == qR[m];
-        flat = __all_sync(0xffffffffu, eq || !ifok);
-        dense_normal<D, IXY>(a, qL, qR, L, R, ifok, al, amdq, apdq, roe);
-    }
-
-    // ---------------- CFL, limiter, second-order corrections ----------------
-    if (lim) {
-        const double c = fabs(dtn) * D::top_speed(roe);     // the largest of dtn s and -dtn s over the waves
-        cflm = cflm > c ? cflm : c;
-    }
-    double bmL[MEQN], bpL[MEQN], bmR[MEQN], bpR[MEQN];
-#pragma unroll
-    for (int m = 0; m < MEQN; m++) { cqxx[m] = 0.0; bmL[m] = 0.0; bpL[m] = 0.0; bmR[m] = 0.0; bpR[m] = 0.0; }
-    if (!flat) {                                   // a line of one state carries no waves
-        if (a.order == 2) {
-            double dr[MW], dl[MW];
-            if (a.limit_any) {
-                double alr[MW], roer[NR];
-#pragma unroll
-                for (int p = 0; p < MW; p++) alr[p] = ctx.shfl_down(al[p]);
-#pragma unroll
-                for (int r = 0; r < NR; r++) roer[r] = r < RP::NROE_WAVE ? ctx.shfl_down(roe[r]) : 0.0;
-                dense_dots<D, IXY>(al, roe, alr, roer, dr);
-#pragma unroll
-                for (int p = 0; p < MW; p++) dl[p] = ctx.shfl_up(dr[p]);
-            }
-            dense_correct<D, IXY>(a, al, roe, dr, dl, dtn, lim, cqxx);
+        for (int m = 0; m < MEQN; m++) {
+            A[m] = cor ? amdq[m] + cqxx[m] : amdq[m];
+            Pf[m] = cor ? apdq[m] - cqxx[m] : apdq[m];
         }
-        // ---------------- transverse splits ----------------
-        if (a.trans > 0) {
-            const bool cor = a.order == 2 && a.trans == 2;
-            double A[MEQN], Pf[MEQN];
-#pragma unroll
-            for (int m = 0; m < MEQN; m++) {
-                A[m] = cor ? amdq[m] + cqxx[m] : amdq[m];
-                Pf[m] = cor ? apdq[m] - cqxx[m] : apdq[m];
-            }
-            const bool sub = __all_sync(0xffffffffu, D::subsonic(roe) || !lim);
-            dense_split<D, IXY>(A, roe, sub, lim, bmL, bpL);
-            dense_split<D, IXY>(Pf, roe, sub, lim, bmR, bpR);
-        }
+        const bool sub = __all_sync(0xffffffffu, D::subsonic(S.roe) || !lim);
+        dense_split<D, IXY>(A, S.roe, sub, lim, bmL, bpL);
+        dense_split<D, IXY>(Pf, S.roe, sub, lim, bmR, bpR);
     }
 #pragma unroll
     for (int m = 0; m < MEQN; m++) fadd[m] = 0.5 * cqxx[m];
@@ -194,10 +256,14 @@ __device__ __forceinline__ void lean_chunk(const StepArgs& a, Ctx& ctx, const do
             C4[m] = dtt * g1;
         }
     }
+    constexpr int NX = SM::NX;
+    const int mine = tid / LANES * T + slot - 1;
+    if (cellok) {
 #pragma unroll
-    for (int m = 0; m < MEQN; m++) {
-        CXb[m * NT + tid] = C0[m];
-        CXb[(MEQN + m) * NT + tid] = C4[m];
+        for (int m = 0; m < MEQN; m++) {
+            CXb[m * NX + mine] = C0[m];
+            CXb[(MEQN + m) * NX + mine] = C4[m];
+        }
     }
     ctx.sync();
 
@@ -205,13 +271,13 @@ __device__ __forceinline__ void lean_chunk(const StepArgs& a, Ctx& ctx, const do
     if (cellok) {
         auto qx = [&](int m, int kk, int ll) -> double& {
             const int ci = IXY == 1 ? kk : ll, cj = IXY == 1 ? ll : kk;
-            return Qx[(m * TY + (cj - j0)) * SM::QP + (ci - i0)];
+            return Qx[(m * T + (cj - j0)) * SM::QP + (ci - i0)];
         };
         auto qi = [&](int m, int kk, int ll) -> double { return IXY == 1 ? hq(m, kk, ll) : qx(m, kk, ll); };
         auto in_tile_line = [&](int ll) {
-            return IXY == 1 ? (ll >= j0 && ll < j0 + TY && ll < a.my) : (ll >= i0 && ll < i0 + TX && ll < a.mx);
+            return IXY == 1 ? (ll >= j0 && ll < j0 + T && ll < a.my) : (ll >= i0 && ll < i0 + T && ll < a.mx);
         };
-        const int up = tid - 32, dn = tid + 32;     // the lanes of lines line-1 and line+1
+        const int up = mine - T, dn = mine + T;         // the lanes of lines line-1 and line+1
         if (in_tile_line(line)) {
 #pragma unroll
             for (int m = 0; m < MEQN; m++) {
@@ -219,7 +285,7 @@ __device__ __forceinline__ void lean_chunk(const StepArgs& a, Ctx& ctx, const do
                 if (line == cfirst) v = qx(m, k, line);                 // has up(line-1) already
                 else {
                     v = qi(m, k, line);
-                    if (trans) v = v + CXb[m * NT + up];
+                    if (trans) v = v + CXb[m * NX + up];
                 }
                 if (IXY == 1) {
                     v = v + C1[m] - C2[m];
@@ -227,7 +293,7 @@ __device__ __forceinline__ void lean_chunk(const StepArgs& a, Ctx& ctx, const do
                 } else {
                     v = v + (trans ? (C1[m] - C2[m] - C3[m]) : (C1[m] - C2[m]));
                 }
-                if (trans && line != clast) v = v - CXb[(MEQN + m) * NT + dn];
+                if (trans && line != clast) v = v - CXb[(MEQN + m) * NX + dn];
                 qx(m, k, line) = v;
             }
         }
@@ -246,11 +312,11 @@ __device__ __forceinline__ void lean_chunk(const StepArgs& a, Ctx& ctx, const do
     }
 }
 
-// True in every thread when the tile's input halo (rows j0-2..j0+TY+1,
-// columns i0-2..i0+TX+1, clipped to the ghosted array: every cell either sweep
+// True in every thread when the tile's input halo (rows j0-2..j0+T+1,
+// columns i0-2..i0+T+1, clipped to the ghosted array: every cell either sweep
 // reads) holds one state.  A NaN never compares equal, so a non-finite halo
 // is never uniform.
-template <class RP, int TX, int TY, int TR>
+template <class RP, int TR>
 __device__ __forceinline__ bool lean_uniform_halo(const StepArgs& a, const double* H, int i0, int j0, int tid, int nt)
 {
     constexpr int MEQN = RP::MEQN;
@@ -261,8 +327,8 @@ __device__ __forceinline__ bool lean_uniform_halo(const StepArgs& a, const doubl
     bool same = true;
     // columns c, c+1 (c even) sit side by side in the swizzled box: one
     // 16-byte load per pair
-    for (int e = tid; e < TR * 16; e += nt) {
-        const int r = e >> 4, c = (e & 15) * 2;
+    for (int e = tid; e < TR * (TR / 2); e += nt) {
+        const int r = e / (TR / 2), c = (e % (TR / 2)) * 2;
         if (r <= rmax && c <= cmax) {
 #pragma unroll
             for (int m = 0; m < MEQN; m++) {
@@ -276,33 +342,48 @@ __device__ __forceinline__ bool lean_uniform_halo(const StepArgs& a, const doubl
 
 // The two sweeps of the full tile step over the staged halo H; returns this
 // thread's running CFL maximum.
-template <class RP, int TX, int TY, int NT, class Ctx>
-__device__ __forceinline__ double lean_tile_sweeps(const StepArgs& a, Ctx& ctx, const double* H, double* Qx, double* CX,
-                                                   int i0, int j0, double dtdx, double dtdy)
+template <class RP, int T, int NT, bool SPLIT, class Ctx>
+__device__ __forceinline__ double lean_tile_sweeps(const StepArgs& a, Ctx& ctx, double* H, double* Qx, double* CX, int i0,
+                                                   int j0, double dtdx, double dtdy)
 {
     constexpr int MEQN = RP::MEQN;
-    constexpr int LPC = NT / 32;
-    const int warp = ctx.tid() >> 5;
+    using SM = LeanSmem<RP, T, NT, SPLIT>;
+    constexpr int LPC = SM::LPC;
+    const int mine = ctx.tid() / (T + 4);
     double cflm = 0.0;
-    int chunk = 0;
-    {
-        const int first = j0 - 1;
-        const int last = (j0 + TY < a.my) ? j0 + TY : a.my;
-        for (int c0 = first; c0 <= last; c0 += LPC, chunk++) {
-            const int line = c0 + warp;
-            const int clast = (c0 + LPC - 1 < last) ? c0 + LPC - 1 : last;
-            lean_chunk<RP, 1, TX, TY, NT>(a, ctx, H, Qx, CX + (chunk & 1) * 2 * MEQN * NT, i0, j0, line, c0, clast,
-                                          line <= last, dtdx, dtdy, cflm);
+    if constexpr (SPLIT) {
+        // rows of the halo, each by itself; then the tile's columns of the swept
+        // rows, and the ghost columns beside it
+        const int first = j0 - 2, last = j0 + T + 1 < a.my + 1 ? j0 + T + 1 : a.my + 1;
+        for (int c0 = first; c0 <= last; c0 += LPC) {
+            const int line = c0 + mine;
+            lean_split_line<RP, 1, T, NT>(a, ctx, H, Qx, i0, j0, line < last ? line : last, line <= last, true, dtdx, cflm);
         }
-    }
-    {
-        const int first = i0 - 1;
-        const int last = (i0 + TX < a.mx) ? i0 + TX : a.mx;
-        for (int c0 = first; c0 <= last; c0 += LPC, chunk++) {
-            const int line = c0 + warp;
-            const int clast = (c0 + LPC - 1 < last) ? c0 + LPC - 1 : last;
-            lean_chunk<RP, 2, TX, TY, NT>(a, ctx, H, Qx, CX + (chunk & 1) * 2 * MEQN * NT, i0, j0, line, c0, clast,
-                                          line <= last, dtdy, dtdx, cflm);
+        ctx.sync();
+        const int own = i0 + T < a.mx ? i0 + T : a.mx;
+        const int yfirst = i0 == 0 ? -2 : i0, ylast = own == a.mx ? a.mx + 1 : own - 1;
+        for (int c0 = yfirst; c0 <= ylast; c0 += LPC) {
+            const int line = c0 + mine;
+            lean_split_line<RP, 2, T, NT>(a, ctx, H, Qx, i0, j0, line < ylast ? line : ylast, line <= ylast,
+                                          line >= 0 && line < own, dtdy, cflm);
+        }
+    } else {
+        int chunk = 0;
+        {
+            const int first = j0 - 1, last = j0 + T < a.my ? j0 + T : a.my;
+            for (int c0 = first; c0 <= last; c0 += LPC, chunk++) {
+                const int line = c0 + mine, clast = c0 + LPC - 1 < last ? c0 + LPC - 1 : last;
+                lean_chunk<RP, 1, T, NT>(a, ctx, H, Qx, CX + (chunk & 1) * 2 * MEQN * SM::NX, i0, j0, line < last ? line : last,
+                                         c0, clast, line <= last, dtdx, dtdy, cflm);
+            }
+        }
+        {
+            const int first = i0 - 1, last = i0 + T < a.mx ? i0 + T : a.mx;
+            for (int c0 = first; c0 <= last; c0 += LPC, chunk++) {
+                const int line = c0 + mine, clast = c0 + LPC - 1 < last ? c0 + LPC - 1 : last;
+                lean_chunk<RP, 2, T, NT>(a, ctx, H, Qx, CX + (chunk & 1) * 2 * MEQN * SM::NX, i0, j0, line < last ? line : last,
+                                         c0, clast, line <= last, dtdy, dtdx, cflm);
+            }
         }
     }
     return cflm;
@@ -317,13 +398,12 @@ __device__ __forceinline__ double lean_tile_sweeps(const StepArgs& a, Ctx& ctx, 
 // tile whose copy does not arrive reports a timeout instead of a result.
 constexpr long long kTmaWaitCycles = 2000000000LL;
 
-template <class RP, int TX, int TY, int NT, class Ctx>
+template <class RP, int T, int NT, bool SPLIT, class Ctx>
 __device__ __forceinline__ void lean_tile_at(const StepArgs& a, Ctx& ctx, const TileId& tile, const CUtensorMap* tm0,
                                              const CUtensorMap* tm1, uint64_t* bar)
 {
     constexpr int MEQN = RP::MEQN;
-    using SM = LeanSmem<RP, TX, TY, NT>;
-    static_assert(TX + 4 <= 32 && TY + 4 <= 32, "a line's cells i0-2 .. i0+TX+1 must fit its 32 lanes");
+    using SM = LeanSmem<RP, T, NT, SPLIT>;
     static_assert(RP::MAUX == 0, "the lean body serves the solvers without aux arrays");
     double* H = ctx.smem();
     {
@@ -334,7 +414,7 @@ __device__ __forceinline__ void lean_tile_at(const StepArgs& a, Ctx& ctx, const 
     double* CX = Qx + SM::QX;
     double* red = CX + SM::CX;
     const int tid = ctx.tid();
-    const int i0 = tile.bx * TX, j0 = tile.by * TY;
+    const int i0 = tile.bx * T, j0 = tile.by * T;
     double* qout = a.qout;
     double dt = a.dt;
     const CUtensorMap* tm = tm0;
@@ -350,8 +430,8 @@ __device__ __forceinline__ void lean_tile_at(const StepArgs& a, Ctx& ctx, const 
     if (tid == 0) {
         mbar_init(bar, 1);
         mbar_arrive_expect_tx(bar, (uint32_t)(SM::HS * 8 + a.halo_shortfall));
-        tma_load_3d(H, tm, bar, i0, j0, 0);
-        tma_load_3d(H + SM::BOX, tm, bar, i0 + 16, j0, 0);
+#pragma unroll
+        for (int b = 0; b < SM::NBOX; b++) tma_load_3d(H + b * SM::BOX, tm, bar, i0 + 16 * b, j0, 0);
     }
     const double dtdx = dt / a.dx, dtdy = dt / a.dy;
     double cflm = 0.0;
@@ -361,7 +441,7 @@ __device__ __forceinline__ void lean_tile_at(const StepArgs& a, Ctx& ctx, const 
     bool keep = false;                             // the tile's cells keep their values
     if (fault) {
         mbar_wait_bounded(bar, 0, kTmaWaitCycles);  // let a late copy land before the CTA moves on
-    } else if (lean_uniform_halo<RP, TX, TY, SM::TR>(a, H, i0, j0, tid, NT)) {
+    } else if (lean_uniform_halo<RP, SM::TR>(a, H, i0, j0, tid, NT)) {
         // A tile whose input halo holds one state has zero waves and
         // fluctuations at every interface: its cells keep their values (the
         // full step adds only zeros) and only its CFL number is computed.
@@ -371,17 +451,19 @@ __device__ __forceinline__ void lean_tile_at(const StepArgs& a, Ctx& ctx, const 
         bool finite = true;
         const double cu = uniform_cfl<RP>(q0, a.prm, dtdx, dtdy, finite);
         if (finite) {                              // the same in every thread
-            for (int e = tid; e < TY * SM::QP; e += NT) {
+            for (int e = tid; e < T * SM::QP; e += NT) {
 #pragma unroll
-                for (int m = 0; m < MEQN; m++) Qx[m * TY * SM::QP + e] = q0[m];
+                for (int m = 0; m < MEQN; m++) Qx[m * T * SM::QP + e] = q0[m];
             }
             cflm = cu;
             keep = true;
         }
     }
-    if (!fault && !keep) cflm = lean_tile_sweeps<RP, TX, TY, NT>(a, ctx, H, Qx, CX, i0, j0, dtdx, dtdy);
+    if (!fault && !keep) cflm = lean_tile_sweeps<RP, T, NT, SPLIT>(a, ctx, H, Qx, CX, i0, j0, dtdx, dtdy);
     ctx.sync();
-    finish_tile<MEQN, TX, TY, NT, SM::QP>(a, ctx, tile, Qx, TY * SM::QP, red, qout, i0, j0, cflm, dt, fault);
+    bool bad = false;
+    if (!fault) bad = store_tile<MEQN, T, T, NT, SM::QP>(a, ctx, Qx, T * SM::QP, qout, i0, j0, dt);
+    report_cell<NT>(a, ctx, tile.ntiles, red, cflm, bad, fault);
 }
 
 }  // namespace claw2

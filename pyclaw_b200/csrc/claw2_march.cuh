@@ -422,29 +422,8 @@ __device__ __forceinline__ bool march_y(const StepArgs& a, const MarchJob& J, co
     return top >= 0x7ff00000u;
 }
 
-// The CTA's CFL maximum, and in the last CTA to arrive the step's: CFL numbers
-// are >= 0, so their bits order as integers and one atomic maximum per CTA
-// collects them in the cell that a.partials points to (zero between launches);
-// a non-finite state counts as infinity.  No scratch grows with the tiles.
-__device__ __forceinline__ void march_report(const StepArgs& a, DevCtx& ctx, int ntiles, double cflm, bool bad)
-{
-    const bool nf = __syncthreads_or(bad || cflm != cflm);
-    const double mw = ctx.warp_max(cflm);           // the x warp's, in thread 0
-    if (threadIdx.x != 0) return;
-    unsigned long long* cell = reinterpret_cast<unsigned long long*>(a.partials);
-    constexpr unsigned long long inf = 0x7ff0000000000000ULL;
-    atomicMax(cell, nf ? inf : (unsigned long long)__double_as_longlong(mw));
-    __threadfence();
-    if (atomicAdd(a.ticket, 1u) != (unsigned)(ntiles - 1)) return;
-    __threadfence();
-    const unsigned long long top = atomicExch(cell, 0ULL);
-    *a.ticket = 0u;
-    finish_step(a, ctx, top >= inf ? 0.0 : __longlong_as_double((long long)top), top >= inf ? 1 : 0);
-    __threadfence();
-}
-
 // One CTA's tile: MARCH_TX columns by up to `rows` rows.  CELL: the CFL maximum
-// is collected by march_report, else by report_cfl through one partial per tile.
+// is collected by collect_cfl, else by report_cfl through one partial per tile.
 template <class RP, bool CELL>
 __device__ __forceinline__ void march_tile(const StepArgs& a, const TileId& tile, int rows)
 {
@@ -488,7 +467,11 @@ __device__ __forceinline__ void march_tile(const StepArgs& a, const TileId& tile
     } else {
         bad = march_y<L>(a, J, ring, qin, qout);
     }
-    if constexpr (CELL) march_report(a, ctx, tile.ntiles, cflm, bad);
+    if constexpr (CELL) {
+        const bool nf = __syncthreads_or(bad || cflm != cflm);
+        const double mw = ctx.warp_max(cflm);      // the x warp's, in thread 0
+        if (threadIdx.x == 0) collect_cfl(a, ctx, tile.ntiles, mw, nf, false);
+    }
     else report_cfl<MARCH_NT>(a, ctx, tile, red, cflm, bad, false);
 }
 

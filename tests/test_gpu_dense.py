@@ -9,10 +9,13 @@ are zero, subnormal or far smaller than the density, states outside 2^-100 ..
 2^100, regions of one state next to a jump, limiters that differ by wave.  The
 tolerance is therefore none (a zero's sign aside, which == does not see).
 """
+import ctypes
+
 import numpy as np
 import pytest
 
 import gpu_helpers as H
+from pyclaw_b200 import _lib
 
 pytestmark = pytest.mark.gpu
 
@@ -89,3 +92,37 @@ def test_states(orc, name, mode, order, kind):
 def test_limiters(orc, name, mode, lim):
     p = H.problem(name, 45, 33, mode, mthlim=lim[:H.SOLVERS[name]["num_waves"]])
     check(orc, p, data("transonic", p, 8), 0.3)
+
+
+# 28-cell tiles: one CTA per SM (147 and 128 tiles), two per SM (303 and 602)
+@pytest.mark.parametrize("name", NAMES)
+@pytest.mark.parametrize("mode", [2, -1])
+@pytest.mark.parametrize("shape", [(29, 2030), (1790, 56), (57, 2802), (8401, 29)])
+def test_large_tile_edges(orc, name, mode, shape):
+    p = H.problem(name, shape[0], shape[1], mode, bcl=(2, 1), bcu=(2, 3))
+    check(orc, p, data("transonic", p, 1), 0.3, steps=2)
+
+
+@pytest.mark.parametrize("name", NAMES)
+def test_split_step_of_buffers_off_16_bytes(orc, name):
+    """The halo copies need 16-byte boundaries; split, other buffers are stepped
+    by the general body."""
+    t, lib = H.torch(), _lib.load()
+    p = H.problem(name, 61, 40, -1)
+    qbc = orc.new_qbc(p, data("transonic", p, 4))
+    orc.fill_ghosts(p, qbc)
+    L = _lib.layout(p)
+    src = H.to_dev(p, qbc, L)
+    qin, qout = t.empty(src.numel() + 1, dtype=t.float64, device="cuda")[1:], t.empty_like(src)
+    qin.copy_(src)
+    scratch = t.zeros(lib.claw2_scratch_bytes(ctypes.byref(p)), dtype=t.uint8, device="cuda")
+    cfl = t.zeros(1, dtype=t.float64, device="cuda")
+    dt = 1e-3
+    rc = lib.claw2_step(ctypes.byref(p), ctypes.c_void_p(qin.data_ptr()), ctypes.c_void_p(qout.data_ptr()), None, dt,
+                        ctypes.c_void_p(scratch.data_ptr()), ctypes.c_void_p(cfl.data_ptr()), H.stream())
+    assert rc == 0
+    got = H.from_dev(p, qout, p.num_eqn, L)
+    ref = orc.step_hyperbolic(p, qbc, None, dt)
+    orc.fill_ghosts(p, qbc)
+    assert np.array_equal(got, qbc)
+    assert float(cfl.item()) == ref
