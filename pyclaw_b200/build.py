@@ -4,9 +4,10 @@
 
 Compiles the sources under csrc/ (claw2_capi.cu: the plain step and the C ABI;
 claw2_acoustics.cu: the unsplit acoustics step; claw2_lean.cu: the Euler and
-shallow-water step; claw2_batch.cu: the batched form; claw2_adjoint.cu: multi-shot acoustics and its adjoint) with nvcc for
-sm_100a only, without FMA contraction so that the step keeps the reference's
-rounding, as objects compiled in parallel under pyclaw_b200/_build/, and links
+shallow-water step; claw2_psystem.cu: the unsplit p-system step; claw2_batch.cu:
+the batched form; claw2_adjoint.cu: multi-shot acoustics and its adjoint) with
+nvcc for sm_100a only, without FMA contraction so that the step keeps the
+reference's rounding, as objects compiled in parallel under pyclaw_b200/_build/, and links
 them into pyclaw_b200/libclaw2.so (in-tree, so the library travels with the
 source tree).
 """
@@ -22,6 +23,7 @@ SRCS = [os.path.join(HERE, "csrc", "claw2_capi.cu"),
         os.path.join(HERE, "csrc", "claw2_batch.cu"),
         os.path.join(HERE, "csrc", "claw2_acoustics.cu"),
         os.path.join(HERE, "csrc", "claw2_lean.cu"),
+        os.path.join(HERE, "csrc", "claw2_psystem.cu"),
         os.path.join(HERE, "csrc", "claw2_adjoint.cu")]
 OBJDIR = os.path.join(HERE, "_build")
 DEPS = SRCS + [os.path.join(HERE, "csrc", "claw2_kernels.cuh"),
@@ -35,6 +37,7 @@ DEPS = SRCS + [os.path.join(HERE, "csrc", "claw2_kernels.cuh"),
                os.path.join(HERE, "csrc", "claw2_launch.cuh"),
                os.path.join(HERE, "csrc", "claw2_host.h"),
                os.path.join(HERE, "csrc", "claw2_lean.cuh"),
+               os.path.join(HERE, "csrc", "claw2_psystem.cuh"),
                os.path.join(HERE, "csrc", "claw2_tma.cuh"),
                os.path.join(ROOT, "include", "claw2.h"),
                os.path.join(ROOT, "include", "claw2_adjoint.h")]

@@ -289,8 +289,9 @@ int launch_step_t(const StepArgs& a, int nbx, int nby, cudaStream_t st, bool cha
 // device loop, so this step may overlap its end (launch_kernel).
 int launch_step(const claw2_problem* p, const StepArgs& a, cudaStream_t st, bool chained = false)
 {
-    if (march_body(p)) return launch_march(p->rp, a, st, chained);
     const bool split = p->transverse < 0;
+    if (march_body(p)) return launch_march(p->rp, a, st, chained);
+    if (p->rp == CLAW2_RP_PSYSTEM && p->use_fwave && p->index_capa < 0 && !split) return launch_psystem(a, st, chained);
     // the lean body's halo copies start on 16-byte boundaries; other buffers keep
     // the general split body (unsplit they are refused)
     const uintptr_t start = a.ctrl ? reinterpret_cast<uintptr_t>(a.q0) | reinterpret_cast<uintptr_t>(a.q1)

@@ -53,4 +53,8 @@ int launch_march(int rp, const StepArgs& a, cudaStream_t st, bool chained);
 constexpr int LEAN_T = 28;             // edge of its large tiles
 int launch_lean(int rp, bool split, const StepArgs& a, cudaStream_t st, bool chained);
 
+// The unsplit step of the p-system with f-waves and no capacity (claw2_psystem.cuh,
+// claw2_psystem.cu).
+int launch_psystem(const StepArgs& a, cudaStream_t st, bool chained);
+
 }  // namespace claw2
