@@ -3,7 +3,7 @@
     python -m pyclaw_b200.build          # or pyclaw_b200.build.build()
 
 Compiles the sources under csrc/ (claw2_capi.cu: the plain step and the C ABI;
-claw2_acoustics.cu: the unsplit acoustics step; claw2_lean.cu: the Euler and
+claw2_acoustics.cu: the acoustics step; claw2_lean.cu: the Euler and
 shallow-water step; claw2_psystem.cu: the unsplit p-system step; claw2_batch.cu:
 the batched form; claw2_adjoint.cu: multi-shot acoustics and its adjoint) with
 nvcc for sm_100a only, without FMA contraction so that the step keeps the
@@ -31,6 +31,7 @@ DEPS = SRCS + [os.path.join(HERE, "csrc", "claw2_kernels.cuh"),
                os.path.join(HERE, "csrc", "claw2_riemann.cuh"),
                os.path.join(HERE, "csrc", "claw2_light.cuh"),
                os.path.join(HERE, "csrc", "claw2_march.cuh"),
+               os.path.join(HERE, "csrc", "claw2_rows.cuh"),
                os.path.join(HERE, "csrc", "claw2_dense.cuh"),
                os.path.join(HERE, "csrc", "claw2_exact.cuh"),
                os.path.join(HERE, "csrc", "claw2_limit.cuh"),

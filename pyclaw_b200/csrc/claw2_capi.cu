@@ -219,11 +219,11 @@ using namespace claw2;
 // ===========================================================================
 namespace {
 
-// Problems stepped by the marching body (launch_step): the unsplit acoustics
-// solvers without capacity or f-waves.
+// Problems stepped by the marching body, split by the row body (launch_step): the
+// acoustics solvers without capacity or f-waves.
 bool march_body(const claw2_problem* p)
 {
-    return p->transverse >= 0 && p->index_capa < 0 && !p->use_fwave &&
+    return p->index_capa < 0 && !p->use_fwave &&
            (p->rp == CLAW2_RP_ACOUSTICS || p->rp == CLAW2_RP_VC_ACOUSTICS);
 }
 
@@ -248,7 +248,7 @@ void tiles(const claw2_problem* p, int* nbx, int* nby)
     const bool split = p->transverse < 0;
     int tx = split ? STX : UTX, ty = split ? STY : UTY;
     // the marching body counts in tiles only for the scratch it is given
-    if (march_body(p) && march_small_grid(p->mx, p->my)) tx = ty = MARCH_SMALL_TILE;
+    if (!split && march_body(p) && march_small_grid(p->mx, p->my)) tx = ty = MARCH_SMALL_TILE;
     // as does the lean body
     if (lean_body(p)) tx = ty = LEAN_T;
     *nbx = (p->mx + tx - 1) / tx;
@@ -290,7 +290,7 @@ int launch_step_t(const StepArgs& a, int nbx, int nby, cudaStream_t st, bool cha
 int launch_step(const claw2_problem* p, const StepArgs& a, cudaStream_t st, bool chained = false)
 {
     const bool split = p->transverse < 0;
-    if (march_body(p)) return launch_march(p->rp, a, st, chained);
+    if (march_body(p)) return split ? launch_rows(p->rp, a, st, chained) : launch_march(p->rp, a, st, chained);
     if (p->rp == CLAW2_RP_PSYSTEM && p->use_fwave && p->index_capa < 0 && !split) return launch_psystem(a, st, chained);
     // the lean body's halo copies start on 16-byte boundaries; other buffers keep
     // the general split body (unsplit they are refused)

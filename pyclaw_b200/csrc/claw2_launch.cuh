@@ -48,6 +48,9 @@ int launch_kernel(void (*kern)(KArgs...), dim3 grid, int threads, int smem, cuda
 int march_rows_per_cta(int rp, long long cols, int my);
 int launch_march(int rp, const StepArgs& a, cudaStream_t st, bool chained);
 
+// The split acoustics step (claw2_rows.cuh, claw2_acoustics.cu).
+int launch_rows(int rp, const StepArgs& a, cudaStream_t st, bool chained);
+
 // The step of the Euler and shallow-water solvers (claw2_lean.cuh,
 // claw2_lean.cu); the state buffers start on 16-byte boundaries.
 constexpr int LEAN_T = 28;             // edge of its large tiles
