@@ -186,7 +186,7 @@ CLAW2_EXPORT int claw2_step(const claw2_problem* p, const double* q_in, double* 
  * waits for `bytes` (a multiple of 8, at most 65536; 0 restores normal
  * operation) more than its halo copies deliver, so its wait on the copies runs
  * out after about a second; the step then reports CLAW2_ERR_TIMEOUT through
- * the controller (a NaN CFL number without one) and writes no cells. */
+ * the controller (a NaN CFL number without one) and such CTAs write no cells. */
 CLAW2_EXPORT int claw2_debug_halo_shortfall(int bytes);
 
 /* claw2_step without any device allocation, for callers that may not allocate

@@ -51,6 +51,7 @@ struct StepArgs {
     double dx, dy, dt;
     int order, trans, capa, fwave, limit_any;
     int mthlim[CLAW2_MAX_WAVES];
+    int* list;             // tiles left to step (lean_scan_tile), their number in the scratch header, or null
     int limit_first;       // limiter of the first min(waves, 4) waves if they share it, else -1
     double prm[CLAW2_MAX_PARAMS];
     int ghost_fused;
@@ -923,6 +924,9 @@ struct DevCtx {
 // per CTA collects them in the cell that a.partials points to (zero between
 // launches); a non-finite state counts as infinity, a tile that could not be
 // computed as more.  No scratch grows with the tiles.
+// LIST_WORD: word of the scratch header with the number of listed tiles (zero
+// between launches).
+constexpr int LIST_WORD = 4;
 __device__ __forceinline__ void collect_cfl(const StepArgs& a, DevCtx& ctx, int ntiles, double cfl, bool nonfinite, bool fault)
 {
     unsigned long long* cell = reinterpret_cast<unsigned long long*>(a.partials);
@@ -933,6 +937,7 @@ __device__ __forceinline__ void collect_cfl(const StepArgs& a, DevCtx& ctx, int 
     __threadfence();
     const unsigned long long top = atomicExch(cell, 0ULL);
     *a.ticket = 0u;
+    a.ticket[LIST_WORD] = 0u;
     finish_step(a, ctx, top >= inf ? 0.0 : __longlong_as_double((long long)top), top >= lost ? 2 : top >= inf ? 1 : 0);
     __threadfence();
 }

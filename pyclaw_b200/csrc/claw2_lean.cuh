@@ -34,9 +34,10 @@
 //    of 16 columns x T+4 rows x MEQN fields, 128-byte swizzle; see
 //    claw2_tma.cuh) while the threads wait on an mbarrier; x lines read rows
 //    of it and y lines read down its columns;
-//  - a tile whose staged halo holds one state skips both sweeps: every
-//    interface would join two equal states, so its cells keep their values
-//    and its CFL number comes from one Riemann solve (uniform_cfl).
+//  - a tile whose halo holds one state skips both sweeps: every interface
+//    would join two equal states, so its cells keep their values and its CFL
+//    number comes from one Riemann solve (uniform_cfl).  On large grids a pass
+//    of its own looks for such tiles (lean_scan_tile).
 //
 // Bound by the latency of the FP64 chains and by issue: 128 registers a thread
 // leave 4 warps per SM quarter, which issue 44% of the cycles (FP64 pipe 36%
@@ -45,12 +46,12 @@
 // against 280, split 197 against 175).  us a step on a B200, before (the solves
 // of claw2_riemann.cuh; split, the general body; 28-tiles only) and now:
 //                     64 x 48      256^2        641 x 163    1500^2
-//   Euler 4 unsplit   36.5  15.3   36.7  29.4   36.8  30.4   331  280
-//   Euler 4 split     44.5  12.3   47.9  23.2   49.9  23.3   394  175
-//   Euler 5 unsplit   40.0  17.0   40.0  34.1   40.0  34.5   532  368
-//   Euler 5 split     47.8  13.9   48.9  25.4   49.2  25.6   697  214
-//   shallow unsplit   25.8  12.2   26.4  21.1   26.6  22.3   367  282
-//   shallow split     29.5  10.2   31.5  16.3   32.7  18.4   275  184
+//   Euler 4 unsplit   36.5  15.3   36.7  28.1   36.8  29.0   331  262
+//   Euler 4 split     44.5  12.3   47.9  22.6   49.9  23.0   394  177
+//   Euler 5 unsplit   40.0  17.0   40.0  32.5   40.0  33.0   532  314
+//   Euler 5 split     47.8  13.9   48.9  24.7   49.2  25.3   697  215
+//   shallow unsplit   25.8  12.2   26.4  20.6   26.6  22.0   367  290
+//   shallow split     29.5  10.2   31.5  15.9   32.7  18.0   275  187
 #pragma once
 
 #include "claw2_dense.cuh"
@@ -389,18 +390,76 @@ __device__ __forceinline__ double lean_tile_sweeps(const StepArgs& a, Ctx& ctx, 
     return cflm;
 }
 
-// Whole-tile unsplit step with the lean body (the caller checks that the
-// problem has no capacity function and no f-waves).  tm0 / tm1: tensor maps
-// of the input state (uncontrolled mode: both of a.qin; controlled mode: of
-// a.q0 and a.q1) over the ghosted planes (mx+4 x my+4 x MEQN, row pitch ld,
-// 16 x 32 x MEQN boxes, 128-byte swizzle); bar: an mbarrier in shared memory.
-// The halo copy is waited for at most about a second (clock64 cycles); a
-// tile whose copy does not arrive reports a timeout instead of a result.
+// One warp's look at a tile of a large grid: a tile whose input halo holds one
+// state gets its values, ghost images and CFL number here (as in lean_tiles; the
+// caller checks that there is no source term), any other is listed for lean_tiles.
+// A lane reads a column of the halo, some rows at a time; the first difference ends
+// it.  Bound by HBM: 4096^2 cells of shallow water at rest 191 us, 830 MB at 4.3 TB/s.
+// Returns the tile's CFL number, infinity for a state that is not finite, 0 for a
+// listed tile.
+template <class RP, int T>
+__device__ __forceinline__ double lean_scan_tile(const StepArgs& a, const double* __restrict__ qin, double* __restrict__ qout,
+                                                 int tile, double dtdx, double dtdy)
+{
+    constexpr int MEQN = RP::MEQN;
+    static_assert(T + 4 == 32, "a lane per column");
+    const int lane = threadIdx.x & 31, nbx = (a.mx + T - 1) / T, i0 = tile % nbx * T, j0 = tile / nbx * T;
+    const int cmax = a.mx + 3 - i0, rmax = a.my + 3 - j0 < 31 ? a.my + 3 - j0 : 31;
+    const double* p = qin + (long long)j0 * a.ld + (i0 + (lane < cmax ? lane : cmax));
+    double q0[MEQN];
+#pragma unroll
+    for (int m = 0; m < MEQN; m++) q0[m] = __shfl_sync(0xffffffffu, p[m * a.plane], 0);
+    bool keep = true;
+    constexpr int ROWS = MEQN == 3 ? 8 : 4;
+    for (int r = 0; r <= rmax && keep; r += ROWS) {
+        bool same = true;
+#pragma unroll
+        for (int k = 0; k < ROWS; k++) {
+            const long long o = (long long)(r + k < rmax ? r + k : rmax) * a.ld;
+#pragma unroll
+            for (int m = 0; m < MEQN; m++) same = same & (p[o + m * a.plane] == q0[m]);
+        }
+        keep = __all_sync(0xffffffffu, same);
+    }
+    double cu = 0.0;
+    if (keep) cu = uniform_cfl<RP>(q0, a.prm, dtdx, dtdy, keep);       // the same in every lane
+    if (!keep) {
+        if (lane == 0) a.list[atomicAdd(a.ticket + LIST_WORD, 1u)] = tile;
+        return 0.0;
+    }
+    const int i = i0 - 2 + lane, n = a.my - j0 < T ? a.my - j0 : T;
+    if (lane >= 2 && lane < 2 + T && i < a.mx) {
+        double* d = qout + (long long)(j0 + 2) * a.ld + (i + CLAW2_NUM_GHOST);
+        for (int r = 0; r < n; r++, d += a.ld) {
+#pragma unroll
+            for (int m = 0; m < MEQN; m++) d[m * a.plane] = q0[m];
+        }
+        const bool edge = i0 <= 1 || i0 + T >= a.mx - 2 || j0 <= 1 || j0 + T >= a.my - 2;
+        if (a.ghost_fused && edge) {
+            for (int j = j0; j < j0 + n; j++)
+                if (i <= 1 || i >= a.mx - 2 || j <= 1 || j >= a.my - 2) write_ghosts<MEQN>(a, qout, i, j, q0);
+        }
+    }
+    bool finite = true;
+#pragma unroll
+    for (int m = 0; m < MEQN; m++) finite = finite && isfinite(q0[m]);
+    return finite ? cu : __longlong_as_double(0x7ff0000000000000LL);
+}
+
+// The step of a CTA's tiles (the caller checks that the problem has no capacity
+// function and no f-waves): tile blockIdx.x of the grid, or with LISTED every
+// gridDim.x-th of the list.  LOOK: one-state tiles are passed over.  tm0 / tm1:
+// tensor maps of the input state (uncontrolled mode: both of a.qin; controlled
+// mode: of a.q0 and a.q1) over the ghosted planes (mx+4 x my+4 x MEQN, row pitch
+// ld, boxes of 16 x (T+4) x MEQN, 128-byte swizzle); bar: an mbarrier in shared
+// memory.  The halo copy is waited for at most about a second (clock64 cycles); a
+// tile whose copy does not arrive reports a timeout instead of a result, and its
+// CTA steps no further ones.
 constexpr long long kTmaWaitCycles = 2000000000LL;
 
-template <class RP, int T, int NT, bool SPLIT, class Ctx>
-__device__ __forceinline__ void lean_tile_at(const StepArgs& a, Ctx& ctx, const TileId& tile, const CUtensorMap* tm0,
-                                             const CUtensorMap* tm1, uint64_t* bar)
+template <class RP, int T, int NT, bool SPLIT, bool LOOK, bool LISTED, class Ctx>
+__device__ __forceinline__ void lean_tiles(const StepArgs& a, Ctx& ctx, const CUtensorMap* tm0, const CUtensorMap* tm1,
+                                           uint64_t* bar)
 {
     constexpr int MEQN = RP::MEQN;
     using SM = LeanSmem<RP, T, NT, SPLIT>;
@@ -414,56 +473,72 @@ __device__ __forceinline__ void lean_tile_at(const StepArgs& a, Ctx& ctx, const 
     double* CX = Qx + SM::QX;
     double* red = CX + SM::CX;
     const int tid = ctx.tid();
-    const int i0 = tile.bx * T, j0 = tile.by * T;
     double* qout = a.qout;
     double dt = a.dt;
     const CUtensorMap* tm = tm0;
     if (a.ctrl) {
-        if (a.ctrl->done) return;                  // uniform across the grid
+        const int done = a.ctrl->done, cur = a.ctrl->cur;           // loaded together
         dt = a.ctrl->dt;
-        const int cur = a.ctrl->cur;
+        if (done) return;                          // uniform across the grid
         tm = cur ? tm1 : tm0;
         qout = cur ? a.q0 : a.q1;
     }
-    // stage the halo: rows j0-2.., columns i0-2.. are ghosted-array indices
-    // j0, i0 (x = i0 is even, so the box starts on a 16-byte boundary)
-    if (tid == 0) {
-        mbar_init(bar, 1);
-        mbar_arrive_expect_tx(bar, (uint32_t)(SM::HS * 8 + a.halo_shortfall));
-#pragma unroll
-        for (int b = 0; b < SM::NBOX; b++) tma_load_3d(H + b * SM::BOX, tm, bar, i0 + 16 * b, j0, 0);
-    }
+    const int nbx = (a.mx + T - 1) / T, ncta = gridDim.x;
+    const int count = LISTED ? *(volatile int*)(a.ticket + LIST_WORD) : ncta;
+    // CTAs that report: those with a tile, or the first if there is none
+    const int reports = count < ncta ? (count > 0 ? count : 1) : ncta;
+    if (LISTED && (int)blockIdx.x >= reports) return;
     const double dtdx = dt / a.dx, dtdy = dt / a.dy;
+    if (tid == 0) mbar_init(bar, 1);
     double cflm = 0.0;
-    ctx.sync();                                    // the barrier is initialised
-    // the whole CTA takes the same path
-    const bool fault = __syncthreads_or(!mbar_wait_bounded(bar, 0, kTmaWaitCycles));
-    bool keep = false;                             // the tile's cells keep their values
-    if (fault) {
-        mbar_wait_bounded(bar, 0, kTmaWaitCycles);  // let a late copy land before the CTA moves on
-    } else if (lean_uniform_halo<RP, SM::TR>(a, H, i0, j0, tid, NT)) {
-        // A tile whose input halo holds one state has zero waves and
-        // fluctuations at every interface: its cells keep their values (the
-        // full step adds only zeros) and only its CFL number is computed.
-        double q0[MEQN];
+    bool bad = false, fault = false;
+    uint32_t phase = 0;
+    for (int b = blockIdx.x; b < count; b += ncta) {
+        const int tile = LISTED ? a.list[b] : b, i0 = tile % nbx * T, j0 = tile / nbx * T;
+        // stage the halo: rows j0-2.., columns i0-2.. are ghosted-array indices
+        // j0, i0 (x = i0 is even, so the box starts on a 16-byte boundary)
+        if (tid == 0) {
+            mbar_arrive_expect_tx(bar, (uint32_t)(SM::HS * 8 + a.halo_shortfall));
 #pragma unroll
-        for (int m = 0; m < MEQN; m++) q0[m] = H[lean_hidx<MEQN, SM::TR>(m, 0, 0)];
-        bool finite = true;
-        const double cu = uniform_cfl<RP>(q0, a.prm, dtdx, dtdy, finite);
-        if (finite) {                              // the same in every thread
-            for (int e = tid; e < T * SM::QP; e += NT) {
-#pragma unroll
-                for (int m = 0; m < MEQN; m++) Qx[m * T * SM::QP + e] = q0[m];
-            }
-            cflm = cu;
-            keep = true;
+            for (int k = 0; k < SM::NBOX; k++) tma_load_3d(H + k * SM::BOX, tm, bar, i0 + 16 * k, j0, 0);
         }
+        ctx.sync();                                // the barrier is initialised
+        // the whole CTA takes the same path
+        fault = __syncthreads_or(!mbar_wait_bounded(bar, phase, kTmaWaitCycles));
+        if (fault) {
+            mbar_wait_bounded(bar, phase, kTmaWaitCycles);       // let a late copy land before the CTA moves on
+            break;
+        }
+        bool keep = false;                         // the tile's cells keep their values
+        if (LOOK && lean_uniform_halo<RP, SM::TR>(a, H, i0, j0, tid, NT)) {
+            // A tile whose input halo holds one state has zero waves and
+            // fluctuations at every interface: its cells keep their values (the
+            // full step adds only zeros) and only its CFL number is computed.
+            double q0[MEQN];
+#pragma unroll
+            for (int m = 0; m < MEQN; m++) q0[m] = H[lean_hidx<MEQN, SM::TR>(m, 0, 0)];
+            keep = true;
+            const double cu = uniform_cfl<RP>(q0, a.prm, dtdx, dtdy, keep);
+            if (keep) {                            // the same in every thread
+                for (int e = tid; e < T * SM::QP; e += NT) {
+#pragma unroll
+                    for (int m = 0; m < MEQN; m++) Qx[m * T * SM::QP + e] = q0[m];
+                }
+                cflm = cflm > cu ? cflm : cu;
+            }
+        }
+        if (!keep) {
+            const double c = lean_tile_sweeps<RP, T, NT, SPLIT>(a, ctx, H, Qx, CX, i0, j0, dtdx, dtdy);
+            cflm = cflm > c || cflm != cflm ? cflm : c;          // a NaN stays
+        }
+        // (the split sweeps wrote to the halo that the next copy overwrites)
+        if (LISTED && SPLIT) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        ctx.sync();
+        bad |= store_tile<MEQN, T, T, NT, SM::QP>(a, ctx, Qx, T * SM::QP, qout, i0, j0, dt);
+        if (!LISTED) break;
+        phase ^= 1;
     }
-    if (!fault && !keep) cflm = lean_tile_sweeps<RP, T, NT, SPLIT>(a, ctx, H, Qx, CX, i0, j0, dtdx, dtdy);
-    ctx.sync();
-    bool bad = false;
-    if (!fault) bad = store_tile<MEQN, T, T, NT, SM::QP>(a, ctx, Qx, T * SM::QP, qout, i0, j0, dt);
-    report_cell<NT>(a, ctx, tile.ntiles, red, cflm, bad, fault);
+    report_cell<NT>(a, ctx, reports, red, cflm, bad, fault);
 }
 
 }  // namespace claw2

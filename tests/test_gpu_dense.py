@@ -126,3 +126,45 @@ def test_split_step_of_buffers_off_16_bytes(orc, name):
     orc.fill_ghosts(p, qbc)
     assert np.array_equal(got, qbc)
     assert float(cfl.item()) == ref
+
+
+# more than 16 tiles of 28 cells per SM: one-state tiles are stepped by a pass of their own
+@pytest.mark.parametrize("name", NAMES)
+@pytest.mark.parametrize("mode", [2, -1])
+@pytest.mark.parametrize("kind", ["jump", "rest", "transonic"])
+@pytest.mark.parametrize("shape,bcs", [((66401, 5), ((1, 3), (3, 1))), ((30, 33199), ((2, 2), (2, 2)))])
+def test_listed_tiles(orc, name, mode, kind, shape, bcs):
+    p = H.problem(name, shape[0], shape[1], mode, bcl=bcs[0], bcu=bcs[1])
+    q = data("column" if kind == "rest" else kind, p, 2)
+    if kind == "rest":                     # every tile holds the one state
+        q[:] = q[:, :1, :1]
+    check(orc, p, q, 0.3, steps=1)
+
+
+@pytest.mark.parametrize("name,mode", [("euler5", 2), ("shallow", 2), ("euler4", -1)])
+def test_listed_steps_in_one_call_equal_single_calls(name, mode):
+    from pyclaw_b200 import _abi
+    from pyclaw_b200.device import DeviceState
+    t, lib = H.torch(), _lib.load()
+    p = H.problem(name, 1400, 1400, mode, bcl=(1, 3), bcu=(3, 1))
+    q = data("jump", p, 6)
+    results = []
+    for calls in (1, 8):
+        dev = DeviceState(p)
+        dev.upload_q(q)
+        c = _abi.Control.from_address(dev.ctrl_host.data_ptr())
+        _lib.check(lib.claw2_control_init(ctypes.byref(c), 0.0, 0.2 / 1400, 1e9, 1.0, 0.9, 1e99, 1, 0, 1 << 40, 0.9),
+                   "claw2_control_init")
+        dev.ctrl.copy_(dev.ctrl_host)
+        for _ in range(calls):
+            _lib.check(lib.claw2_advance(ctypes.byref(p), dev.ptr(dev.q[0]), dev.ptr(dev.q[1]), dev.ptr(dev.aux),
+                                         dev.ptr(dev.ctrl), dev.ptr(dev.scratch), 8 // calls, dev.stream), "claw2_advance")
+        dev.ctrl_host.copy_(dev.ctrl)
+        t.cuda.synchronize()
+        c = _abi.Control.from_address(dev.ctrl_host.data_ptr())
+        assert c.numsteps == 8 and c.error == 0
+        assert not dev.scratch[:64].any()
+        dev.cur = c.cur
+        results.append((dev.download_q(), c.t, c.dt))
+    assert results[0][1:] == results[1][1:]
+    assert np.array_equal(results[0][0], results[1][0])
