@@ -168,6 +168,7 @@ __global__ void halo_kernel(double* q0, double* q1, const claw2_control* c, doub
 __global__ void aux_from_q_kernel(double* aux, const double* q0, const double* q1, const claw2_control* c,
                                   long long plane, int from, int to)
 {
+    chain_wait();
     if (c->done) return;
     const double* q = (c->cur ? q1 : q0) + (long long)from * plane;
     double* d = aux + (long long)to * plane;
@@ -181,6 +182,7 @@ __global__ void gauge_record_kernel(claw2_gauges g, const double* q0, const doub
                                     int meqn, long long ld, long long plane, int mx, int my)
 {
     __shared__ int row;
+    chain_wait();
     if (threadIdx.x == 0) {
         row = -1;
         if (c->numsteps != g.state[1]) {
@@ -233,6 +235,14 @@ bool lean_body(const claw2_problem* p)
 {
     return p->index_capa < 0 && !p->use_fwave &&
            (p->rp == CLAW2_RP_EULER_4WAVE || p->rp == CLAW2_RP_EULER_5WAVE || p->rp == CLAW2_RP_SHALLOW_ROE);
+}
+
+// Arguments of a step whose ghost cells the caller does not fill himself: beside
+// custom sides the tile bodies write them too (the marching body does not).
+void step_args(const claw2_problem* p, double* q, StepArgs& a)
+{
+    fill_args(p, q, a);
+    if (!a.ghost_fused && fused_beside_custom(p) && !(march_body(p) && p->transverse >= 0)) a.ghost_fused = a.custom = 1;
 }
 
 // The tiles that claw2_scratch_bytes counts for it: 29x29 cells, 13x13 on
@@ -461,7 +471,7 @@ int claw2_step(const claw2_problem* p, const double* q_in, double* q_out, const 
     if (rc) return rc;
     if (!q_in || !q_out || !scratch || !cfl_dev || (p->num_aux > 0 && !aux) || q_in == q_out) return CLAW2_ERR_INVALID;
     StepArgs a;
-    fill_args(p, q_out, a);
+    step_args(p, q_out, a);
     a.qin = q_in; a.qout = q_out; a.aux = aux; a.dt = dt;
     set_scratch(scratch, a);
     a.cfl_out = cfl_dev;
@@ -478,7 +488,7 @@ int claw2_advance(const claw2_problem* p, double* q0, double* q1, const double* 
     if (rc) return rc;
     if (!q0 || !q1 || !ctrl || !scratch || (p->num_aux > 0 && !aux) || nsteps < 0) return CLAW2_ERR_INVALID;
     StepArgs a;
-    fill_args(p, q0, a);
+    step_args(p, q0, a);
     a.q0 = q0; a.q1 = q1; a.aux = aux; a.ctrl = ctrl;
     set_scratch(scratch, a);
     for (int n = 0; n < nsteps; n++) {
@@ -515,15 +525,24 @@ int apply_hooks(const claw2_problem* p, const claw2_hooks* hooks, StepArgs& a)
     return CLAW2_OK;
 }
 
-int launch_aux_from_q(const claw2_hooks* hooks, const StepArgs& a, double* aux, double* q0, double* q1,
-                      claw2_control* ctrl, cudaStream_t st)
+// One step of a loop with hooks (or gauges, hooks null then).  chained: the previous
+// operation in the stream is a step or gauge kernel of the same loop; the kernels here
+// wait for the one before them themselves (chain_wait).
+int launch_hooked(const claw2_problem* p, const claw2_hooks* hooks, const StepArgs& a, double* aux, bool chained,
+                  cudaStream_t st)
 {
-    if (!hooks || hooks->aux_from_q == 0) return CLAW2_OK;
-    const long long n = a.plane;
-    int blocks = (int)((n + 255) / 256);
-    if (blocks > 148 * 8) blocks = 148 * 8;
-    aux_from_q_kernel<<<blocks, 256, 0, st>>>(aux, q0, q1, ctrl, a.plane, hooks->aux_q - 1, hooks->aux_from_q - 1);
-    return cudaGetLastError() == cudaSuccess ? CLAW2_OK : CLAW2_ERR_CUDA;
+    int rc;
+    if (hooks && hooks->aux_from_q != 0) {
+        int blocks = (int)((a.plane + 255) / 256);
+        if (blocks > 148 * 8) blocks = 148 * 8;
+        if ((rc = launch_kernel(aux_from_q_kernel, dim3(blocks), 256, 0, st, chained, aux, (const double*)a.q0,
+                                (const double*)a.q1, (const claw2_control*)a.ctrl, a.plane, hooks->aux_q - 1,
+                                hooks->aux_from_q - 1)))
+            return rc;
+        chained = true;
+    }
+    if ((rc = launch_step(p, a, st, chained)) || a.ghost_fused) return rc;
+    return launch_fill(p, nullptr, p->num_eqn, p->bc_lower, p->bc_upper, false, a.q0, a.q1, a.ctrl, st);
 }
 }  // namespace
 
@@ -536,17 +555,12 @@ int claw2_advance_hooked(const claw2_problem* p, double* q0, double* q1, const d
     if (rc) return rc;
     if (!q0 || !q1 || !ctrl || !scratch || !hooks || (p->num_aux > 0 && !aux) || nsteps < 0) return CLAW2_ERR_INVALID;
     StepArgs a;
-    fill_args(p, q0, a);
+    step_args(p, q0, a);
     a.q0 = q0; a.q1 = q1; a.aux = aux; a.ctrl = ctrl;
     set_scratch(scratch, a);
     if ((rc = apply_hooks(p, hooks, a))) return rc;
-    for (int n = 0; n < nsteps; n++) {
-        if ((rc = launch_aux_from_q(hooks, a, const_cast<double*>(aux), q0, q1, ctrl, S(stream)))) return rc;
-        if ((rc = launch_step(p, a, S(stream)))) return rc;
-        if (!a.ghost_fused &&
-            (rc = launch_fill(p, nullptr, p->num_eqn, p->bc_lower, p->bc_upper, false, q0, q1, ctrl, S(stream))))
-            return rc;
-    }
+    for (int n = 0; n < nsteps; n++)
+        if ((rc = launch_hooked(p, hooks, a, const_cast<double*>(aux), n > 0 && a.ghost_fused, S(stream)))) return rc;
     return CLAW2_OK;
 }
 
@@ -558,19 +572,17 @@ int claw2_advance_gauged(const claw2_problem* p, double* q0, double* q1, const d
     if (!q0 || !q1 || !ctrl || !scratch || !g || (p->num_aux > 0 && !aux) || nsteps < 0) return CLAW2_ERR_INVALID;
     if (g->ngauges < 1 || g->capacity < 1 || !g->cells || !g->record || !g->state) return CLAW2_ERR_INVALID;
     StepArgs a;
-    fill_args(p, q0, a);
+    step_args(p, q0, a);
     a.q0 = q0; a.q1 = q1; a.aux = aux; a.ctrl = ctrl;
     set_scratch(scratch, a);
     if (hooks && (rc = apply_hooks(p, hooks, a))) return rc;
     const int threads = 128;
     for (int n = 0; n < nsteps; n++) {
-        if ((rc = launch_aux_from_q(hooks, a, const_cast<double*>(aux), q0, q1, ctrl, S(stream)))) return rc;
-        if ((rc = launch_step(p, a, S(stream)))) return rc;
-        if (!a.ghost_fused &&
-            (rc = launch_fill(p, nullptr, p->num_eqn, p->bc_lower, p->bc_upper, false, q0, q1, ctrl, S(stream))))
+        if ((rc = launch_hooked(p, hooks, a, const_cast<double*>(aux), n > 0, S(stream)))) return rc;
+        if ((rc = launch_kernel(gauge_record_kernel, dim3(1), threads, 0, S(stream), a.ghost_fused, *g,
+                                (const double*)q0, (const double*)q1, (const claw2_control*)ctrl, (int)p->num_eqn, a.ld, a.plane,
+                                (int)p->mx, (int)p->my)))
             return rc;
-        gauge_record_kernel<<<1, threads, 0, S(stream)>>>(*g, q0, q1, ctrl, p->num_eqn, a.ld, a.plane, p->mx, p->my);
-        if (cudaGetLastError() != cudaSuccess) return CLAW2_ERR_CUDA;
     }
     return CLAW2_OK;
 }

@@ -36,6 +36,15 @@ inline bool fused_ghosts(const claw2_problem* p)
     return p->mx >= 4 && p->my >= 4;
 }
 
+// Custom sides do not keep a tile body from writing the other sides' ghost cells
+// (write_custom_corners has the corners beside them).
+inline bool fused_beside_custom(const claw2_problem* p)
+{
+    for (int d = 0; d < 2; d++)
+        if (!periodic_ok(p->bc_lower[d], p->bc_upper[d])) return false;
+    return p->mx >= 4 && p->my >= 4;
+}
+
 inline void fill_args(const claw2_problem* p, double* q, StepArgs& a)
 {
     claw2_layout L;

@@ -54,7 +54,8 @@ struct StepArgs {
     int* list;             // tiles left to step (lean_scan_tile), their number in the scratch header, or null
     int limit_first;       // limiter of the first min(waves, 4) waves if they share it, else -1
     double prm[CLAW2_MAX_PARAMS];
-    int ghost_fused;
+    int ghost_fused;       // the step writes the ghost cells that are images of its cells
+    int custom;            // with custom sides among them: write_custom_corners
     int bcl[2], bcu[2];
     int src, src_aux;      // source term fused into the final write (claw2_source)
     int ctrl_readonly;     // controlled mode that reports the CFL (cfl_out, +inf if
@@ -680,6 +681,31 @@ CLAW2_HD void euler_radial_source(double (&v)[MEQN], double rad, double gamma1, 
     }
 }
 
+// Corner ghost cells beside a custom side: a side that is not custom takes its
+// ghost cells along a custom side's from that side's ghost cells (fill_kernel's
+// passes over all rows and columns), which no step writes.  tid: 4 MEQN threads of
+// the CTA (or lanes of the warp) that owns the corner's cell.
+template <int MEQN>
+CLAW2_HD void write_custom_corners(const StepArgs& a, double* qo, int i0, int j0, int tx, int ty, int tid)
+{
+    if (tid >= 4 * MEQN) return;
+    const int gx = tid & 1, gy = (tid >> 1) & 1, m = tid >> 2;
+    for (int c = 0; c < 4; c++) {
+        const int ux = c & 1, uy = c >> 1;                          // upper side along x, y
+        if (ux ? i0 + tx < a.mx : i0 > 0) continue;
+        if (uy ? j0 + ty < a.my : j0 > 0) continue;
+        const int bx = ux ? a.bcu[0] : a.bcl[0], by = uy ? a.bcu[1] : a.bcl[1];
+        if ((bx == CLAW2_BC_CUSTOM) == (by == CLAW2_BC_CUSTOM)) continue;
+        const int gi = ux ? a.mx + gx : -1 - gx, gj = uy ? a.my + gy : -1 - gy;
+        const bool alongx = by == CLAW2_BC_CUSTOM;                  // the axis of the side that is not custom
+        const int n = alongx ? a.mx : a.my, g = alongx ? gx : gy, up = alongx ? ux : uy, bc = alongx ? bx : by;
+        const int src = bc == CLAW2_BC_EXTRAP ? (up ? n - 1 : 0) : bc == CLAW2_BC_PERIODIC ? (up ? g : n - 1 - g)
+                                                                                          : (up ? n - 1 - g : g);
+        const double v = qo[qoff(a, m, alongx ? src : gi, alongx ? gj : src)];
+        qo[qoff(a, m, gi, gj)] = bc == CLAW2_BC_WALL && m == (alongx ? 1 : 2) ? -v : v;
+    }
+}
+
 // Write a tile's final values and the ghost cells that are images of them;
 // whether this thread saw one that is not finite.  QP: row pitch of Qx in doubles
 // (TX unless the body pads its rows).
@@ -724,6 +750,7 @@ CLAW2_HD bool store_tile(const StepArgs& a, Ctx& ctx, const double* Qx, int QSTR
             cell_value(ci, cj, i, j, v);
             write_ghosts<MEQN>(a, qout, i, j, v);
         }
+        if (a.custom) write_custom_corners<MEQN>(a, qout, i0, j0, TX, TY, tid);
     }
     return bad != 0;
 }

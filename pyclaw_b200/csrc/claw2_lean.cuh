@@ -428,6 +428,7 @@ __device__ __forceinline__ double lean_scan_tile(const StepArgs& a, const double
         return 0.0;
     }
     const int i = i0 - 2 + lane, n = a.my - j0 < T ? a.my - j0 : T;
+    if (a.custom) write_custom_corners<MEQN>(a, qout, i0, j0, T, T, lane);
     if (lane >= 2 && lane < 2 + T && i < a.mx) {
         double* d = qout + (long long)(j0 + 2) * a.ld + (i + CLAW2_NUM_GHOST);
         for (int r = 0; r < n; r++, d += a.ld) {
