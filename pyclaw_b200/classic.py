@@ -240,6 +240,23 @@ class ClawSolver2D(ClawSolver):
                 return None
         return h
 
+    def _fixed_sides(self, state):
+        """values[axis][0 lower, 1 upper] of the custom sides for
+        DeviceState.set_fixed_sides (None: not custom), or None when the host
+        has to fill them: another callback (a subclass may do anything), one
+        attached to the side opposite to its own, a wrong number of values."""
+        from .hooks import FixedStateBC
+        sides = [[None, None], [None, None]]
+        for k, (side, bcs, fn) in enumerate((("lower", self.bc_lower, self.user_bc_lower),
+                                             ("upper", self.bc_upper, self.user_bc_upper))):
+            for axis in range(2):
+                if bcs[axis] != BC.custom:
+                    continue
+                if type(fn) is not FixedStateBC or fn.side != side or fn.values.shape != (state.num_eqn,):
+                    return None
+                sides[axis][k] = np.ascontiguousarray(fn.values)
+        return sides
+
     def _device_loop_ok(self, solution):
         return self._device_hooks() is not None
 
@@ -270,11 +287,15 @@ class ClawSolver2D(ClawSolver):
                 # fixed-state sides: set once in both state buffers; the
                 # step never writes the ghost cells of custom sides
                 dev = self._dev
-                qbc = dev.ghosted_ref()
-                self._fill_host_bcs(state, qbc, self.bc_lower, self.bc_upper, self.user_bc_lower,
-                                    self.user_bc_upper, negate=True)
-                dev.set_ghosted_ref(qbc, dev.cur)
-                dev.set_ghosted_ref(qbc, 1 - dev.cur)
+                sides = self._fixed_sides(state)
+                if sides is not None:
+                    dev.set_fixed_sides(sides)
+                else:
+                    qbc = dev.ghosted_ref()
+                    self._fill_host_bcs(state, qbc, self.bc_lower, self.bc_upper, self.user_bc_lower,
+                                        self.user_bc_upper, negate=True)
+                    dev.set_ghosted_ref(qbc, dev.cur)
+                    dev.set_ghosted_ref(qbc, 1 - dev.cur)
         gauges = [(int(g[0]), int(g[1])) for g in state.grid.gauges]
         on_gauges = None
         if gauges:

@@ -133,6 +133,29 @@ class DeviceState(object):
         src = torch.from_numpy(np.ascontiguousarray(np.asarray(qbc).transpose(0, 2, 1)))
         self.qview(k)[:, :, :self.p.mx + 2 * _abi.NUM_GHOST].copy_(src)
 
+    def set_fixed_sides(self, sides):
+        """Ghost layers of the custom sides held at constant states, on the
+        device, in both buffers: sides[axis][0 lower, 1 upper] is a float64
+        array of num_eqn values, or None for a side that is not custom.  The
+        order is that of the boundary fill: x sides over all rows, then y sides
+        over all columns."""
+        torch = _torch()
+        g, n = _abi.NUM_GHOST, (self.p.mx, self.p.my)
+        vals = [[None if v is None else torch.from_numpy(v).to(self.device)[:, None, None] for v in pair] for pair in sides]
+
+        def fill(k, axis):
+            a = self.qview(k)[:, :, :self.p.mx + 2 * g]
+            for v, at in zip(vals[axis], (0, n[axis] + g)):
+                if v is not None:
+                    a.narrow(2 - axis, at, g).copy_(v)
+        fill(self.cur, 0)
+        _lib.check(self.lib.claw2_fill_ghosts(ctypes.byref(self.p), self.ptr(self.q[self.cur]), self.stream),
+                   "claw2_fill_ghosts")
+        fill(self.cur, 1)
+        # a step writes the other ghost cells of the buffer it steps to
+        fill(1 - self.cur, 0)
+        fill(1 - self.cur, 1)
+
     # ---- stepping ---------------------------------------------------------
     def step(self, dt):
         """One step q[cur] -> q[1-cur] with explicit dt; returns the CFL number."""

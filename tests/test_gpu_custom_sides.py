@@ -75,3 +75,43 @@ def test_custom_sides_of_the_general_body(orc, sides):
 @pytest.mark.parametrize("sides", SIDES)
 def test_custom_sides_of_listed_tiles(orc, sides):
     run(orc, H.problem("shallow", 66401, 5, 2, bcl=sides[0], bcu=sides[1]), 7)
+
+
+@pytest.mark.parametrize("lower,upper", [((0, 3), (1, 1)), ((1, 0), (3, 1)), ((0, 0), (1, 3)), ((0, 0), (0, 0)), ((0, 2), (1, 2))])
+@pytest.mark.parametrize("solver", ["euler", "acoustics"])
+def test_fixed_sides_set_on_the_device_equal_the_host_fill(solver, lower, upper):
+    import pyclaw_b200 as pc
+
+    class OnHost(pc.hooks.FixedStateBC):
+        """a subclass: the host fills the sides"""
+
+    res = []
+    for cls in (pc.hooks.FixedStateBC, OnHost):
+        domain = pc.Domain([pc.Dimension("x", 0.0, 1.0, 41), pc.Dimension("y", 0.0, 1.0, 30)])
+        st = pc.State(domain, 4 if solver == "euler" else 3)
+        rng = np.random.default_rng(3)
+        if solver == "euler":
+            st.problem_data["gamma"], st.problem_data["gamma1"] = 1.4, 0.4
+            st.q[...] = 0.1 * rng.random(st.q.shape)
+            st.q[0] += 1.0
+            st.q[3] += 2.5
+            sol = pc.ClawSolver2D(pc.riemann.rp2_euler_4wave)
+            lo, up = [1.2, 0.3, 0.1, 3.0], [0.9, -0.1, 0.2, 2.2]
+        else:
+            for k, v in dict(rho=1.0, bulk=4.0, cc=2.0, zz=2.0).items():
+                st.problem_data[k] = v
+            st.q[...] = rng.random(st.q.shape)
+            sol = pc.ClawSolver2D(pc.riemann.rp2_acoustics)
+            lo, up = [0.3, 0.1, -0.2], [0.0, 0.2, 0.1]
+        sol.limiters = 4
+        sol.dimensional_split = False
+        sol.dt_initial = 1e-3
+        sol.bc_lower, sol.bc_upper = list(lower), list(upper)
+        sol.user_bc_lower, sol.user_bc_upper = cls(lo, side="lower"), cls(up, side="upper")
+        solution = pc.Solution(st, domain)
+        sol.setup(solution)
+        for t in (0.02, 0.03):
+            sol.evolve_to_time(solution, t)
+        res.append((solution.state.get_q_host().copy(), solution.t, sol.dt))
+    assert res[0][1:] == res[1][1:]
+    assert np.array_equal(res[0][0], res[1][0])
