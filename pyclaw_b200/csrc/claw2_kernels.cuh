@@ -590,10 +590,11 @@ CLAW2_HD void finish_step(const StepArgs& a, Ctx& ctx, double cfl, int nf)
 
 // Block CFL max (deterministic: max is exact) and last-block epilogue: warp max
 // by shuffles, then one value per warp.  CFL numbers are >= 0; a NaN one
-// counts as a non-finite state, and -1 flags a warp that saw one; a tile that
-// could not be computed reports -2.  red: NT/32 + 1 doubles of shared memory.
+// counts as a non-finite state, and -1 flags a warp that saw one.  red: NT/32 + 1
+// doubles of shared memory.  (collect_cfl does it without partials, where the
+// header of the scratch holds the step's maximum.)
 template <int NT, class Ctx>
-CLAW2_HD void report_cfl(const StepArgs& a, Ctx& ctx, const TileId& tile, double* red, double cflm, bool bad, bool fault)
+CLAW2_HD void report_cfl(const StepArgs& a, Ctx& ctx, const TileId& tile, double* red, double cflm, bool bad)
 {
     const int tid = ctx.tid();
     {
@@ -610,7 +611,7 @@ CLAW2_HD void report_cfl(const StepArgs& a, Ctx& ctx, const TileId& tile, double
             if (red[t] < 0.0) nf = 1;
             else mxv = mxv > red[t] ? mxv : red[t];
         }
-        a.partials[tile.part] = fault ? -2.0 : (nf ? -1.0 : mxv);
+        a.partials[tile.part] = nf ? -1.0 : mxv;
         ctx.fence();
         const unsigned int prev = ctx.atomic_inc(a.ticket);
         red[NW] = prev == (unsigned int)(tile.ntiles - 1) ? 1.0 : 0.0;     // this CTA arrived last
@@ -620,25 +621,22 @@ CLAW2_HD void report_cfl(const StepArgs& a, Ctx& ctx, const TileId& tile, double
         // the last CTA reduces every CTA's partial with all its threads
         ctx.fence();
         double cfl = 0.0;
-        bool nonfinite = false, lost = false;
+        bool nonfinite = false;
         for (int b = tid; b < tile.ntiles; b += NT) {
             const double v = ctx.load_volatile(&a.partials[b]);
             if (v < 0.0) nonfinite = true;
             else cfl = cfl > v ? cfl : v;
-            if (v == -2.0) lost = true;
         }
         const bool nfw = ctx.warp_any(nonfinite);
-        const bool lw = ctx.warp_any(lost);
         const double mw = ctx.warp_max(cfl);
-        if ((tid & 31) == 0) red[tid >> 5] = lw ? -2.0 : (nfw ? -1.0 : mw);
+        if ((tid & 31) == 0) red[tid >> 5] = nfw ? -1.0 : mw;
         ctx.sync();
         if (tid == 0) {
             cfl = 0.0;
             int nf = 0;
             for (int t = 0; t < NW; t++) {
-                if (red[t] == -2.0) nf = 2;
-                else if (red[t] < 0.0 && nf == 0) nf = 1;
-                else if (red[t] >= 0.0) cfl = cfl > red[t] ? cfl : red[t];
+                if (red[t] < 0.0) nf = 1;
+                else cfl = cfl > red[t] ? cfl : red[t];
             }
             finish_step(a, ctx, cfl, nf);
             *a.ticket = 0u;
@@ -647,10 +645,6 @@ CLAW2_HD void report_cfl(const StepArgs& a, Ctx& ctx, const TileId& tile, double
     }
 }
 
-// Final values of the tile's cells (Qx: row stride TX, component stride QSTR,
-// row 0 = tile row j0) and their ghost images, then the block CFL max and the
-// last-arriving CTA's reduction over all CTAs (and, in controlled mode, the
-// device-side time-step controller).
 // Geometric source of the Euler equations with radial symmetry (2D, so the
 // factor ndim-1 is 1), two-stage second-order Runge-Kutta step of the
 // reference app (apps/euler_2d/shockbubble.py:89-124), with its operation
@@ -755,15 +749,16 @@ CLAW2_HD bool store_tile(const StepArgs& a, Ctx& ctx, const double* Qx, int QSTR
     return bad != 0;
 }
 
-// fault: the tile could not be computed (its input never arrived): nothing is
-// written and the step reports CLAW2_ERR_TIMEOUT (controlled mode) or a NaN
-// CFL number.
+// Final values of the tile's cells (Qx: row pitch QP, component stride QSTR, row 0 =
+// tile row j0) and their ghost images, then the block CFL max and the
+// last-arriving CTA's reduction over all CTAs (and, in controlled mode, the
+// device-side time-step controller).
 template <int MEQN, int TX, int TY, int NT, int QP = TX, class Ctx>
 CLAW2_HD void finish_tile(const StepArgs& a, Ctx& ctx, const TileId& tile, const double* Qx, int QSTR, double* red,
-                          double* qout, int i0, int j0, double cflm, double dt, bool fault = false)
+                          double* qout, int i0, int j0, double cflm, double dt)
 {
-    const bool bad = !fault && store_tile<MEQN, TX, TY, NT, QP>(a, ctx, Qx, QSTR, qout, i0, j0, dt);
-    report_cfl<NT>(a, ctx, tile, red, cflm, bad, fault);
+    const bool bad = store_tile<MEQN, TX, TY, NT, QP>(a, ctx, Qx, QSTR, qout, i0, j0, dt);
+    report_cfl<NT>(a, ctx, tile, red, cflm, bad);
 }
 
 // f(IntC<0>{}), ..., f(IntC<N-1>{}): a loop whose index is a compile-time constant

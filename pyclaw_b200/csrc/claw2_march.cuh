@@ -472,7 +472,7 @@ __device__ __forceinline__ void march_tile(const StepArgs& a, const TileId& tile
         const double mw = ctx.warp_max(cflm);      // the x warp's, in thread 0
         if (threadIdx.x == 0) collect_cfl(a, ctx, tile.ntiles, mw, nf, false);
     }
-    else report_cfl<MARCH_NT>(a, ctx, tile, red, cflm, bad, false);
+    else report_cfl<MARCH_NT>(a, ctx, tile, red, cflm, bad);
 }
 
 }  // namespace claw2
