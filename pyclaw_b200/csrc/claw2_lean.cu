@@ -131,15 +131,16 @@ int launch_lean_t(const StepArgs& a, cudaStream_t st, bool chained)
 //    beyond the line 641 x 163 35.1 / 30.4 (756); split 12.3 / 23.3, 14.3 / 22.7,
 //    19.6 / 23.7, and 27.4 / 23.3; shallow water 320 x 160 20.7 / 21.1.
 //  - 28 x 28 with 512 threads, one CTA per SM, up to one tile per SM, and for Euler up
-//    to 2: the lowest latency of a wave (641 x 163, 138 tiles, 30.4 us against 50.6
-//    with 256; 500 x 333, 216 tiles, 41 / 53, but shallow water 39.6 / 37.2).  In one
-//    wave the slowest tile decides, so nobody looks for one-state tiles (256 x 256 28.4
-//    against 29.9, 5-wave 32.5 against 35.2).
+//    to 8: the lowest latency of a wave (641 x 163, 138 tiles, 30.4 us against 50.6
+//    with 256; the developed shock bubble of 1280 x 320, 552 tiles of uneven cost, 126
+//    / 153; shallow water 500 x 333, 216 tiles, 39.6 / 37.2).  In one wave the slowest
+//    tile decides, so nobody looks for one-state tiles (256 x 256 28.4 against 29.9,
+//    5-wave 32.5 against 35.2).
 //  - 28 x 28 with 256 threads, two CTAs per SM, beyond: one CTA's waits (its halo
 //    copy, its barriers, the launch of the next CTA) overlap the other's work.
-//    512 / 256 on 800 x 400 60.2 / 58.8, 1500^2 300.9 / 280.4, split 219 / 175,
-//    shallow water 328 / 285.  Not the unsplit 5-wave solver: its spilled
-//    registers miss the L1 that two CTAs' shared memory leaves (373 / 406).
+//    512 / 256 on 1500^2 300.9 / 280.4, split 219 / 175, shallow water 328 / 285.  Not
+//    the unsplit 5-wave solver: its spilled registers miss the L1 that two CTAs'
+//    shared memory leaves (373 / 406).
 //  - from 16 tiles per SM on, a pass of its own (lean_scan_kernel) steps the one-state
 //    tiles and lists the others, whose kernel then holds fewer registers.  Shallow
 //    water 4096^2 at rest around a dam 461 -> 230; no tile at rest, 1500^2: Euler
@@ -158,7 +159,7 @@ int launch_lean_rp(const StepArgs& a, cudaStream_t st, bool chained)
     if (n <= 148) return launch_lean_t<RP, LEAN_T, 512, SPLIT, false, false>(a, st, chained);
     if (n > LIST_TILES && !a.src) return launch_lean_t<RP, LEAN_T, euler && !SPLIT ? 512 : 256, SPLIT, true, false>(a, st, chained);
     if constexpr (euler)
-        if (small_l1 || n <= 2 * 148) return launch_lean_t<RP, LEAN_T, 512, SPLIT, false, true>(a, st, chained);
+        if (small_l1 || n <= 8 * 148) return launch_lean_t<RP, LEAN_T, 512, SPLIT, false, true>(a, st, chained);
     if constexpr (!small_l1) return launch_lean_t<RP, LEAN_T, 256, SPLIT, false, true>(a, st, chained);
     return CLAW2_ERR_INVALID;                      // not reached
 }

@@ -216,8 +216,8 @@ __device__ __forceinline__ void lean_chunk(const StepArgs& a, Ctx& ctx, const do
             Pf[m] = cor ? apdq[m] - cqxx[m] : apdq[m];
         }
         const bool sub = __all_sync(0xffffffffu, D::subsonic(S.roe) || !lim);
-        dense_split<D, IXY>(A, S.roe, sub, lim, bmL, bpL);
-        dense_split<D, IXY>(Pf, S.roe, sub, lim, bmR, bpR);
+        D::template split<IXY>(A, S.roe, sub, bmL, bpL);
+        D::template split<IXY>(Pf, S.roe, sub, bmR, bpR);
     }
 #pragma unroll
     for (int m = 0; m < MEQN; m++) fadd[m] = 0.5 * cqxx[m];

@@ -21,7 +21,7 @@ pytestmark = pytest.mark.gpu
 
 NAMES = ["euler4", "euler5", "shallow"]
 SHAPES = [(4, 4), (27, 5), (28, 3), (29, 28), (56, 29), (57, 61), (85, 4), (4, 40)]
-KINDS = ["transonic", "still", "small", "subnormal", "jump", "column", "high", "low"]
+KINDS = ["transonic", "still", "small", "subnormal", "tails", "jump", "column", "high", "low"]
 
 
 def data(kind, p, seed):
@@ -37,6 +37,9 @@ def data(kind, p, seed):
         u, v = np.zeros((mx, my)), np.zeros((mx, my))
     elif kind == "small":
         u, v = u * 2.0 ** -500, v * 2.0 ** rng.integers(-900, -400, (mx, my)).astype(float)
+    elif kind == "tails":                  # through every binade down to zero, in still gas
+        u, v = 10.0 ** (-330.0 * X) * rng.choice([-1.0, 1.0], (mx, my)), 10.0 ** (-330.0 * Y)
+        rho[:], pr[:] = 1.0, 1.0
     elif kind == "subnormal":
         u, v = rng.integers(-9, 10, (2, mx, my)) * 5e-324
     elif kind in ("jump", "column"):
