@@ -507,10 +507,10 @@ def run_ours(args, world, rank, local):
     alg_bytes = 8 * (2 * prob.num_eqn + prob.num_aux) * cells   # per launch (one step)
     avg_kernel_s = t_dev / args.steps
     achieved = alg_bytes / avg_kernel_s / 1e9
-    rec = _ncu_record("step_kernel_split_euler1280x320" if args.split else "lean_step_kernel_euler1280x320")
+    rec = _ncu_record("lean_step_kernel_split_euler1280x320" if args.split else "lean_step_kernel_euler1280x320")
     traffic = (rec["dram_bytes_read"] + rec["dram_bytes_write"]) if rec else None
-    # FP64 pipe: the step's real bound (about 1,900 FP64 instructions per cell,
-    # IEEE divisions and square roots, no FMA contraction): lane-slots of the
+    # FP64 pipe: the step's real bound (about 1,000 FP64 instructions per cell,
+    # quotients and square roots rounded as IEEE ones, no FMA contraction): lane-slots of the
     # FP64 pipe used per launch (ncu warp instructions x 32) per second, against
     # SMs x 64 FP64 lanes x the SM clock
     fp64 = None
@@ -898,7 +898,7 @@ def run_shallow(args):
 def run_acoustics(args):
     """Config 1: 256^2 constant-coefficient acoustics (walls, unsplit with
     transverse_waves=2, MC, cfl_desired 0.9) from t = 0 to 0.6 through the
-    device-controlled loop (one launch per step, the light tile body); the
+    device-controlled loop (one launch per step, the marching body); the
     whole run is timed with CUDA events, the oracle's OpenMP form times the
     same run on the host cores."""
     import torch
