@@ -44,7 +44,8 @@ struct StepArgs {
     double* q1;
     claw2_control* ctrl;   // controlled mode when non-null
     double* partials;      // one double per CTA
-    unsigned int* ticket;  // block-arrival counter, zero between launches
+    unsigned int* ticket;  // block-arrival counter, zero between launches; with `list` the head of a
+                           // 64-byte header, without one a word whose neighbours may be others' counters
     double* cfl_out;       // uncontrolled mode: CFL number (NaN if the state went non-finite)
     long long ld, plane;
     int mx, my;
@@ -941,7 +942,8 @@ struct DevCtx {
     __device__ __forceinline__ void prefetch_l2(const void* p) const { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 };
 
-// Word of the scratch header with the number of listed tiles (zero between launches).
+// Word of the scratch header with the number of listed tiles (zero between launches);
+// only steps with a list have it (the shots' counters lie next to one another).
 constexpr int LIST_WORD = 4;
 
 // A CTA's CFL maximum (one thread), and in the last CTA to arrive the step's:
@@ -966,7 +968,7 @@ __device__ __forceinline__ void collect_cfl(const StepArgs& a, DevCtx& ctx, int 
     if (arrived != (unsigned)(ntiles - 1)) return;
     const unsigned long long top = atomicExch(cell, 0ULL);
     *a.ticket = 0u;
-    a.ticket[LIST_WORD] = 0u;
+    if (a.list) a.ticket[LIST_WORD] = 0u;
     const double c = top >= inf ? 0.0 : __longlong_as_double((long long)top);
     const int nf = top >= lost ? 2 : top >= inf ? 1 : 0;
     if (own) {
