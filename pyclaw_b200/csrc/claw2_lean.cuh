@@ -355,15 +355,18 @@ __device__ __forceinline__ double lean_tile_sweeps(const StepArgs& a, Ctx& ctx, 
     if constexpr (SPLIT) {
         // rows of the halo, each by itself; then the tile's columns of the swept
         // rows, and the ghost columns beside it
+        // A warp past the last line leaves (`lead`: its first line of a pass): the lines
+        // are rewritten in place, and it would read one that another warp writes.
+        const int lead = ctx.tid() / 32 * (32 / (T + 4));
         const int first = j0 - 2, last = j0 + T + 1 < a.my + 1 ? j0 + T + 1 : a.my + 1;
-        for (int c0 = first; c0 <= last; c0 += LPC) {
+        for (int c0 = first; c0 + lead <= last; c0 += LPC) {
             const int line = c0 + mine;
             lean_split_line<RP, 1, T, NT>(a, ctx, H, Qx, i0, j0, line < last ? line : last, line <= last, true, dtdx, cflm);
         }
         ctx.sync();
         const int own = i0 + T < a.mx ? i0 + T : a.mx;
         const int yfirst = i0 == 0 ? -2 : i0, ylast = own == a.mx ? a.mx + 1 : own - 1;
-        for (int c0 = yfirst; c0 <= ylast; c0 += LPC) {
+        for (int c0 = yfirst; c0 + lead <= ylast; c0 += LPC) {
             const int line = c0 + mine;
             lean_split_line<RP, 2, T, NT>(a, ctx, H, Qx, i0, j0, line < ylast ? line : ylast, line <= ylast,
                                           line >= 0 && line < own, dtdy, cflm);

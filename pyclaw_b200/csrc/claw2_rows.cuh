@@ -120,12 +120,14 @@ __device__ __forceinline__ void rows_tile(const StepArgs& a, DevCtx& ctx, const 
         }
     }
     __syncthreads();
-    const int mine = threadIdx.x / SM::TR;
+    // A warp past the last line leaves its loop (`lead`: its first line of a pass): the
+    // lines are rewritten in place, and it would read one that another warp writes.
+    const int mine = threadIdx.x / SM::TR, lead = threadIdx.x / 32 * (32 / SM::TR);
     double cx = 0.0, cy = 0.0;
     {
         // rows of the halo
         const int first = j0 - 2, last = j0 + T + 1 < a.my + 1 ? j0 + T + 1 : a.my + 1;
-        for (int c0 = first; c0 <= last; c0 += SM::LPC) {
+        for (int c0 = first; c0 + lead <= last; c0 += SM::LPC) {
             const int line = c0 + mine;
             const double t = rows_line<VC, 1, T, NT>(a, J, H, i0, j0, line < last ? line : last, line <= last, true, dtdx);
             cx = cx > t ? cx : t;
@@ -136,7 +138,7 @@ __device__ __forceinline__ void rows_tile(const StepArgs& a, DevCtx& ctx, const 
         // the tile's columns of the swept rows, and the ghost columns beside it
         const int own = i0 + T < a.mx ? i0 + T : a.mx;
         const int first = i0 == 0 ? -2 : i0, last = own == a.mx ? a.mx + 1 : own - 1;
-        for (int c0 = first; c0 <= last; c0 += SM::LPC) {
+        for (int c0 = first; c0 + lead <= last; c0 += SM::LPC) {
             const int line = c0 + mine;
             const double t = rows_line<VC, 2, T, NT>(a, J, H, i0, j0, line < last ? line : last, line <= last,
                                                      line >= 0 && line < own, dtdy);

@@ -13,7 +13,10 @@
 #include <atomic>
 #include <cmath>
 #include <cstdint>
+#include <cstdio>
+#include <cstdlib>
 #include <cstring>
+#include <string>
 #include <thread>
 #include <vector>
 
@@ -23,7 +26,7 @@
 #define __global__
 #define __shared__ static
 #define __forceinline__ inline
-#define __noinline__ __attribute__((noinline))
+#define __noinline__ __attribute__((noinline))      // after the standard headers, which use the name
 
 using std::copysign; using std::fabs; using std::fmax; using std::fmin; using std::isfinite; using std::max; using std::min;
 using std::sqrt;
