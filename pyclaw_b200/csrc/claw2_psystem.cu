@@ -12,24 +12,32 @@
 
 namespace claw2 {
 
-template <int T, int NT>
+// TALL: more rows of tiles than a grid's second dimension holds, in one dimension.
+template <int T, int NT, bool TALL>
 __global__ void __launch_bounds__(NT, 512 / NT) psystem_step_kernel(StepArgs a)
 {
     extern __shared__ double smem_dyn[];
     chain_wait();
     DevCtx ctx{smem_dyn};
-    const TileId t{(int)blockIdx.x, (int)blockIdx.y, (int)gridDim.x, (int)gridDim.y,
-                   (int)(blockIdx.y * gridDim.x + blockIdx.x), (int)(gridDim.x * gridDim.y)};
+    TileId t{(int)blockIdx.x, (int)blockIdx.y, (int)gridDim.x, (int)gridDim.y,
+             (int)(blockIdx.y * gridDim.x + blockIdx.x), (int)(gridDim.x * gridDim.y)};
+    if constexpr (TALL) {
+        t.nbx = (a.mx + T - 1) / T;
+        t.nby = t.ntiles / t.nbx;
+        t.bx = t.part % t.nbx;
+        t.by = t.part / t.nbx;
+    }
     psys_tile<T, NT>(a, ctx, t);
 }
 
-template <int T, int NT>
+template <int T, int NT, bool TALL = false>
 static int launch_psystem_t(const StepArgs& a, cudaStream_t st, bool chained)
 {
-    auto kern = psystem_step_kernel<T, NT>;
+    auto kern = psystem_step_kernel<T, NT, TALL>;
     static std::atomic<uint64_t> optin{0};
     if (smem_optin(optin, kern, PsysSmem<T, NT>::bytes) != cudaSuccess) return CLAW2_ERR_CUDA;
-    return launch_kernel(kern, dim3((a.mx + T - 1) / T, (a.my + T - 1) / T), NT, PsysSmem<T, NT>::bytes, st, chained, a);
+    const int nbx = (a.mx + T - 1) / T, nby = (a.my + T - 1) / T;
+    return launch_kernel(kern, TALL ? dim3(nbx * nby) : dim3(nbx, nby), NT, PsysSmem<T, NT>::bytes, st, chained, a);
 }
 
 // Tiles and block size, as in claw2_lean.cu.  us a step, 12 x 12 / 28 x 28 with 512
@@ -48,6 +56,8 @@ int launch_psystem(const StepArgs& a0, cudaStream_t st, bool chained)
     auto count = [&](int t) { return (long long)((a.mx + t - 1) / t) * ((a.my + t - 1) / t); };
     if (count(12) <= PSYS_SMALL_TILES) return launch_psystem_t<12, 256>(a, st, chained);
     if (count(28) <= PSYS_BIG_BLOCK_TILES) return launch_psystem_t<28, 512>(a, st, chained);
+    // 65535 rows of tiles (one dimension for all: 200 x 200 13.9 us a step instead of 13.6)
+    if (a.my > 65535 * 28) return launch_psystem_t<28, 256, true>(a, st, chained);
     return launch_psystem_t<28, 256>(a, st, chained);
 }
 
