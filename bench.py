@@ -509,10 +509,10 @@ def run_ours(args, world, rank, local):
     achieved = alg_bytes / avg_kernel_s / 1e9
     rec = _ncu_record("lean_step_kernel_split_euler1280x320" if args.split else "lean_step_kernel_euler1280x320")
     traffic = (rec["dram_bytes_read"] + rec["dram_bytes_write"]) if rec else None
-    # FP64 pipe: the step's real bound (about 1,000 FP64 instructions per cell,
-    # quotients and square roots rounded as IEEE ones, no FMA contraction): lane-slots of the
-    # FP64 pipe used per launch (ncu warp instructions x 32) per second, against
-    # SMs x 64 FP64 lanes x the SM clock
+    # FP64 pipe: the step's real bound (quotients and square roots rounded as IEEE
+    # ones, no FMA contraction: 1,240 lane-slots of the FP64 pipe per cell of the
+    # developed flow unsplit, 856 split).  Lane-slots used per launch (ncu warp
+    # instructions x 32) per second, against SMs x 64 FP64 lanes x the SM clock
     fp64 = None
     if rec and rec.get("fp64_pipe_warp_inst"):
         nsm = torch.cuda.get_device_properties(torch.cuda.current_device()).multi_processor_count
