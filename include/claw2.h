@@ -150,8 +150,8 @@ CLAW2_EXPORT const char* claw2_strerror(int status);
  * state.py:176-180; workspace sizes, step2.f90:66-71). */
 CLAW2_EXPORT int claw2_validate(const claw2_problem* p);
 CLAW2_EXPORT int claw2_get_layout(const claw2_problem* p, claw2_layout* out);
-/* Bytes of device scratch (per-block CFL partials) that claw2_step and
- * claw2_advance need. */
+/* Bytes of device scratch that claw2_step and claw2_advance need: a 64-byte header
+ * (arrival counter, CFL maximum) and eight bytes per tile. */
 CLAW2_EXPORT size_t claw2_scratch_bytes(const claw2_problem* p);
 
 /* ---- device-resident path (device layout, device pointers) ----------- */

@@ -251,7 +251,9 @@ void step_args(const claw2_problem* p, double* q, StepArgs& a)
 }
 
 // The tiles that claw2_scratch_bytes counts for it: 29x29 cells, 13x13 on
-// grids of fewer than 148 such tiles.
+// grids of fewer than 148 such tiles.  No kernel has them: like the split acoustics and
+// the p-system bodies, this one needs the header alone.  The count stays, and with it
+// the scratch size and claw2_step_noalloc's largest grid, as callers know them.
 constexpr int MARCH_SMALL_TILE = 13;
 bool march_small_grid(int mx, int my)
 {
@@ -262,16 +264,17 @@ void tiles(const claw2_problem* p, int* nbx, int* nby)
 {
     const bool split = p->transverse < 0;
     int tx = split ? STX : UTX, ty = split ? STY : UTY;
-    // the marching body counts in tiles only for the scratch it is given
+    // (for the scratch size alone)
     if (!split && march_body(p) && march_small_grid(p->mx, p->my)) tx = ty = MARCH_SMALL_TILE;
-    // as does the lean body
+    // the lean body lists its 28-tiles in the scratch
     if (lean_body(p)) tx = ty = LEAN_T;
     *nbx = (p->mx + tx - 1) / tx;
     *nby = (p->my + ty - 1) / ty;
 }
 
-// The scratch of a step: the 64-byte header (the arrival counter) and one
-// CFL partial per tile.
+// The scratch of a step: the 64-byte header (arrival counter, CFL maximum, number of
+// listed tiles) and eight bytes per tile (the generic body's CFL partials, the lean
+// body's list).
 size_t scratch_bytes(const claw2_problem* p)
 {
     int nbx, nby;
@@ -722,8 +725,8 @@ int claw2_graph_destroy(void* graph_exec)
 // memory to its own pool at start-up, a time loop that must not enter the CUDA
 // allocator (an allocation can synchronise the device), or a foreign-language
 // binding that can pass pointers to existing buffers but cannot own device
-// allocations.  claw2_step_noalloc serves them: its scratch (the block-arrival
-// counter and one CFL partial per tile) is the static array below, which every
+// allocations.  claw2_step_noalloc serves them: its scratch (the header and
+// eight bytes per tile, as claw2_scratch_bytes) is the static array below, which every
 // GPU that loads this library holds until the process exits.
 // ---------------------------------------------------------------------------
 }  // extern "C"

@@ -17,8 +17,10 @@
 //    divisions rules that out nearly everywhere (star_subsonic);
 //  - transverse splits where every lane's velocity is subsonic drop the two
 //    terms whose speeds are clipped to zero.
-// An unsplit Euler 4-wave step of 1280 x 320 cells executes 26.9 M warp
-// instructions with them (10.8 M in FP64), 31.0 M (12.0 M) with the plain solves.
+// An unsplit Euler 4-wave step of 1280 x 320 cells, the shock bubble shortly after its
+// start, executes 28.2 M warp instructions with them (11.2 M in FP64; 26.9 M and
+// 10.8 M before low_quot), 31.0 M (12.0 M) with the plain solves.  The developed flow at
+// t = 0.32 takes 37.6 M (15.9 M).
 #pragma once
 
 #include "claw2_exact.cuh"

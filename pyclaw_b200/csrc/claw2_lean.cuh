@@ -46,12 +46,14 @@
 // against 280, split 197 against 175).  us a step on a B200, before (the solves
 // of claw2_riemann.cuh; split, the general body; 28-tiles only) and now:
 //                     64 x 48      256^2        641 x 163    1500^2
-//   Euler 4 unsplit   36.5  15.3   36.7  28.1   36.8  29.0   331  262
-//   Euler 4 split     44.5  12.3   47.9  22.6   49.9  23.0   394  177
-//   Euler 5 unsplit   40.0  17.0   40.0  32.5   40.0  33.0   532  314
-//   Euler 5 split     47.8  13.9   48.9  24.7   49.2  25.3   697  215
-//   shallow unsplit   25.8  12.2   26.4  20.6   26.6  22.0   367  290
-//   shallow split     29.5  10.2   31.5  15.9   32.7  18.0   275  187
+//   Euler 4 unsplit   36.5  14.0   36.7  25.2   36.8  26.6   331  261
+//   Euler 4 split     44.5  11.0   47.9  20.6   49.9  21.7   394  189
+//   Euler 5 unsplit   40.0  15.2   40.0  29.3   40.0  30.7   532  313
+//   Euler 5 split     47.8  12.3   48.9  22.5   49.2  23.7   697  224
+//   shallow unsplit   25.8  10.3   26.4  18.4   26.6  19.5   367  284
+//   shallow split     29.5   8.7   31.5  14.6   32.7  16.1   275  183
+// (1500^2 without still tiles: the pass that looks for them costs the split forms
+// up to 4% there, see launch_lean_rp.)
 #pragma once
 
 #include "claw2_dense.cuh"

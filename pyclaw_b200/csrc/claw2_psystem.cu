@@ -56,7 +56,7 @@ int launch_psystem(const StepArgs& a0, cudaStream_t st, bool chained)
     auto count = [&](int t) { return (long long)((a.mx + t - 1) / t) * ((a.my + t - 1) / t); };
     if (count(12) <= PSYS_SMALL_TILES) return launch_psystem_t<12, 256>(a, st, chained);
     if (count(28) <= PSYS_BIG_BLOCK_TILES) return launch_psystem_t<28, 512>(a, st, chained);
-    // 65535 rows of tiles (one dimension for all: 200 x 200 13.9 us a step instead of 13.6)
+    // 65535 rows of tiles (one dimension for all makes 200 x 200 2% slower)
     if (a.my > 65535 * 28) return launch_psystem_t<28, 256, true>(a, st, chained);
     return launch_psystem_t<28, 256>(a, st, chained);
 }

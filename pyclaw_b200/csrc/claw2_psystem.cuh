@@ -19,9 +19,9 @@
 //  - lines without waves are passed over.
 //
 // Bound by the latency of the FP64 chains (two chunks of lines a step on grids of
-// one wave).  us a step on a B200, the general body and this one: 64 x 48 64 and
-// 11, 200 x 200 68 and 12, 641 x 163 77 and 17, 800 x 400 137 and 36, 1500^2 681
-// and 182.
+// one wave).  us a step on a B200, the general body and this one, with the copy of the
+// strain before it: 64 x 48 64 and 10, 200 x 200 68 and 12, 641 x 163 77 and 18,
+// 800 x 400 137 and 38, 1500^2 681 and 184.
 #pragma once
 
 #include "claw2_exact.cuh"

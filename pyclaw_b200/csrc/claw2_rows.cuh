@@ -16,9 +16,10 @@
 //
 // Bound by the latency of the FP64 chains; 64 registers a thread keep 32 warps on
 // an SM (80 and 24 warps: 73.8 us instead of 68.9 on acoustics 1500^2).  us a step
-// on a B200, the general body and this one: acoustics 64 x 48 19.4 and 7.8, 256^2
-// 22.7 and 10.3, 1280 x 320 37 and 21, 1500^2 169 and 69; variable coefficients
-// 20.8 and 8.1, 25.6 and 10.6, 43 and 23, 205 and 78.
+// on a B200, the general body and this one, a pulse over the whole grid: acoustics
+// 64 x 48 19.4 and 6.2, 256^2 22.7 and 8.5, 1280 x 320 37 and 24, 1500^2 169 and 67;
+// variable coefficients 20.8 and 7.2, 25.6 and 9.5, 43 and 27, 205 and 80.  At rest
+// (lines without waves) 1280 x 320 takes 11 and 12, 1500^2 36 and 45.
 #pragma once
 
 #include "claw2_march.cuh"

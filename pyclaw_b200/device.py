@@ -4,7 +4,7 @@ kernels launched through the C ABI of libclaw2.so on torch's current stream.
 Buffers (device layout of include/claw2.h, ghost cells included):
   q[0], q[1]  ping-pong state buffers; control.cur says which one is current
   aux         auxiliary fields, ghost cells filled once per upload
-  scratch     per-CTA CFL partials + block-arrival counter
+  scratch     arrival counter, CFL maximum, eight bytes per tile
   ctrl        claw2_control (device-side time-step controller)
 """
 import ctypes
