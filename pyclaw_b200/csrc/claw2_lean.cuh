@@ -40,9 +40,9 @@
 //    of its own looks for such tiles (lean_scan_tile).
 //
 // Bound by the latency of the FP64 chains and by issue: 128 registers a thread
-// leave 4 warps per SM quarter, which issue 44% of the cycles (FP64 pipe 36%
-// busy; stalled on dependences 2.1 and barriers 1.4 of the 8 warp-cycles per
-// instruction).  80 registers and 6 warps spill and lose (Euler 1500^2 391 us
+// leave 4 warps per SM quarter, which issue 51% of the cycles (the developed Euler
+// 1280 x 320; FP64 pipe 41% busy; stalled on dependences 1.9 and barriers 0.7 of the
+// 7.7 warp-cycles per instruction).  80 registers and 6 warps spill and lose (Euler 1500^2 391 us
 // against 280, split 197 against 175).  us a step on a B200, before (the solves
 // of claw2_riemann.cuh; split, the general body; 28-tiles only) and now:
 //                     64 x 48      256^2        641 x 163    1500^2
